@@ -194,10 +194,10 @@ __device__ __forceinline__ bool grid_barrier(GridSync* gs, unsigned int nblocks,
     return s_ok != 0;
 }
 
-// Block-wide sum of K doubles; result valid in all threads. blockDim.x must be a
-// multiple of 32 and <= 1024. Fixed shuffle tree: deterministic.
+// Block-wide sum of K doubles, valid in thread 0 only. blockDim.x must be a multiple
+// of 32 and <= 1024. Fixed shuffle tree: deterministic.
 template <int K>
-__device__ __forceinline__ void block_sum(double (&v)[K]) {
+__device__ __forceinline__ void block_sum0(double (&v)[K]) {
     __shared__ double red[32][K];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nw = blockDim.x >> 5;
@@ -205,7 +205,7 @@ __device__ __forceinline__ void block_sum(double (&v)[K]) {
     for (int k = 0; k < K; ++k)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-    __syncthreads();
+    __syncthreads();  // an earlier sum may still read red
     if (lane == 0)
 #pragma unroll
         for (int k = 0; k < K; ++k) red[warp][k] = v[k];
@@ -213,35 +213,44 @@ __device__ __forceinline__ void block_sum(double (&v)[K]) {
     if (warp == 0) {
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            double t = lane < nw ? red[lane][k] : 0.0;
+            v[k] = lane < nw ? red[lane][k] : 0.0;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-            if (lane == 0) red[0][k] = t;
+            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
         }
     }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = red[0][k];
-    __syncthreads();
 }
 
-// Reads the per-block partials part[b*K + k] (b < nblocks) written before the last
-// grid barrier and sums them in a fixed order; every block obtains bit-identical
-// totals. Uses warp 0 of the block; result valid in all threads.
+// Sum of the per-block partials part[b*K + k] (b < nblocks) in a fixed order, valid in
+// thread 0; every block obtains bit-identical totals. Every thread of the block takes
+// its share of the partials, several loads in flight: one warp walking them alone
+// (19 dependent steps for 592 blocks) cost 3 us more after every reduction.
+template <int K>
+__device__ __forceinline__ void grid_sum0(const double* part, int nblocks, double (&t)[K]) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) t[k] = 0.0;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
+        if (K == 2) {
+            const double2 w = __ldcg(reinterpret_cast<const double2*>(part) + b);
+            t[0] += w.x;
+            t[K - 1] += w.y;
+        } else {
+#pragma unroll
+            for (int k = 0; k < K; ++k) t[k] += __ldcg(part + (size_t)b * K + k);
+        }
+    }
+    block_sum0<K>(t);
+}
+
+// grid_sum0 of partials written before the last grid barrier or ticket, valid in all threads.
 template <int K>
 __device__ __forceinline__ void grid_total(const double* part, int nblocks, double (&out)[K]) {
     __shared__ double tot[K];
-    const int lane = threadIdx.x & 31;
-    if (threadIdx.x < 32) {
+    double t[K];
+    grid_sum0<K>(part, nblocks, t);
+    if (threadIdx.x == 0)
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            double t = 0.0;
-            for (int b = lane; b < nblocks; b += 32) t += __ldcg(part + (size_t)b * K + k);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-            if (lane == 0) tot[k] = t;
-        }
-    }
+        for (int k = 0; k < K; ++k) tot[k] = t[k];
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < K; ++k) out[k] = tot[k];
@@ -251,7 +260,7 @@ __device__ __forceinline__ void grid_total(const double* part, int nblocks, doub
 // Block-level partial of K doubles -> part[blockIdx.x*K + k] (thread 0 writes).
 template <int K>
 __device__ __forceinline__ void store_partial(double* part, double (&v)[K]) {
-    block_sum<K>(v);
+    block_sum0<K>(v);
     if (threadIdx.x == 0)
 #pragma unroll
         for (int k = 0; k < K; ++k) __stcg(part + (size_t)blockIdx.x * K + k, v[k]);

@@ -16,7 +16,10 @@
 #include <cstdlib>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <type_traits>
+#include <utility>
 
 #include <cub/cub.cuh>
 
@@ -142,7 +145,8 @@ __global__ void k_qdata(int phys, const double* xyz, const int32_t* conn, const 
         }
         adj3(J, A);
         if (phys == 0) {
-            const double s = k * kQw / fabs(d);
+            // affine elements: 4/5 of the rule's G (ThermalK::apply_affine)
+            const double s = (NQ == 1 ? 0.8 * kQw : kQw) * k / fabs(d);
             double G[6];
             G[0] = s * (A[0][0] * A[0][0] + A[0][1] * A[0][1] + A[0][2] * A[0][2]);
             G[1] = s * (A[0][0] * A[1][0] + A[0][1] * A[1][1] + A[0][2] * A[1][2]);
@@ -228,7 +232,7 @@ __global__ void k_patch_maxinc(const int32_t* __restrict__ pe, const int32_t* __
     __shared__ int s_max;
     const int p = blockIdx.x;
     const int n_el = pe[p + 1] - pe[p];
-    const int nloc = (po[p + 1] - po[p]) + (pf[p + 1] - pf[p]);
+    const int nloc = (po[p + 1] - patch_align(po[p])) + (pf[p + 1] - pf[p]);
     const int nslot = nloc > 0 ? patch_slot(nloc - 1) + 1 : 0;  // lc holds slots
     for (int u = threadIdx.x; u < nslot; u += blockDim.x) cnt[u] = 0;
     if (threadIdx.x == 0) s_max = 0;
@@ -263,7 +267,7 @@ __global__ void k_patch_knorm(const double* __restrict__ qd64, int64_t E, double
         double x[ND], y[ND];
 #pragma unroll
         for (int i = 0; i < ND; ++i) x[i] = i == j ? 1.0 : 0.0;
-        K::apply(qd, kPatchElems, cl, cm, x, y);
+        K::apply(qd, kPatchElems, cl, cm, 1.0, x, y);
 #pragma unroll
         for (int i = 0; i < ND; ++i) rs[i] += fabs(y[i]);
     }
@@ -438,7 +442,7 @@ struct geo_op {
     int n_patches = 0, max_local = 0;
     double nu = 0, cl = 0, cm = 0, cd = 1.0, coef_scalar = 1.0;
     geo::DevBuf<int32_t> eperm, nperm, pe, po, pf, foreign;
-    geo::DevBuf<uint32_t> lc;
+    geo::DevBuf<uint32_t> lc, lc32;
     geo::DevBuf<uint8_t> flags;
     geo::DevBuf<uint8_t> mask_orig;  // Dirichlet mask, original DOF numbering
     geo::DevBuf<double> coef, qd64, g_new, diag_new, dinv64, ediag, diag_orig;
@@ -470,11 +474,11 @@ struct geo_op {
     geo::DevBuf<float> tmp32[2];
     geo::DevBuf<unsigned long long> tmpu[2];
     geo::DevBuf<geo::PcgState> state;
-    geo::DevBuf<double> part;
+    geo::DevBuf<double> part, part_patch;  // per-block partials: node kernels, patch kernel
     geo::PcgState* h_state = nullptr;  // pinned mirror
     int patch_grid[2] = {0, 0};        // resident patch-kernel blocks (FP64, FP32)
     int nbuf[2] = {2, 2};              // element-data buffers of the patch kernel (FP64, FP32)
-    int own_bulk[2] = {0, 0};          // own-node slices by bulk copy (FP32 thermal PCG), see setup
+    int own_bulk[2] = {0, 0};          // own-node slices by bulk copy (PCG), see setup
     size_t patch_smem[2] = {0, 0};     // dynamic shared memory of the patch kernel
     int node_grid[2] = {0, 0};  // resident node-kernel blocks (FP64, mixed)
     // CUDA graphs of PCG iteration chunks, keyed by precision
@@ -496,6 +500,12 @@ inline unsigned nblk(int64_t n, int bs = 256) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, bs), 148 * 64));
 }
 
+// Length of a DOF vector that the patch kernel copies own ranges of, rounded outwards to
+// kNodeAlign nodes: whole 64-entry blocks (sub-arrays of one workspace stay aligned).
+inline size_t padded_dofs(const geo_op* op) {
+    return (size_t)((op->N + kNodeAlign - 1) / kNodeAlign * kNodeAlign * op->dpn + 63) / 64 * 64;
+}
+
 template <class T>
 T* grow(DevBuf<T>& b, size_t n) {
     b.ensure(n);
@@ -514,6 +524,7 @@ PatchView view(const geo_op* op) {
     v.pf = op->pf.p;
     v.foreign = op->foreign.p;
     v.lc = op->lc.p;
+    v.lc32 = op->lc32.p;
     v.flags = op->flags.p;
     v.bound32 = op->pbound32.p;
     v.pfa = op->pfa.p;
@@ -523,22 +534,15 @@ PatchView view(const geo_op* op) {
     v.max_own = op->max_own;
     v.own_bulk = 0;
     v.fslot = op->fslot.p;
-    v.halo = 0;
     v.rec = op->prec.p;
     return v;
 }
 
-// dynamic shared memory of the patch kernel: barriers, element-data buffers, node tables
+// dynamic shared memory of the patch kernel (see patch_smem_bytes)
 template <class K, class T>
-size_t smem_bytes(const geo_op* op, int nbuf, bool own, int halo = 0) {
-    // xs (T), fixed-point accumulators (Scatter<T>::kWords INT32 words), flags (two
-    // tables in the late loop shape), and for PCG the own-node slices
-    const size_t flag_tables = nbuf == 2 ? patch_flag_tables<K, T, 2>() : patch_flag_tables<K, T, 1>();
-    const size_t tables = (size_t)op->max_local * K::DPN * (sizeof(T) + 4 * Scatter<T>::kWords) +
-                          (size_t)op->max_local * flag_tables + 16 +
-                          (own ? (size_t)own_bytes<T>(op->max_own, K::DPN) : 0);
-    return (nbuf == 2 ? patch_smem_tables<K, T, 2>(op->max_for, halo) : patch_smem_tables<K, T, 1>(op->max_for, halo)) +
-           tables;
+size_t smem_bytes(const geo_op* op, int nbuf, bool own, int halo) {
+    return nbuf == 2 ? patch_smem_bytes<K, T, 2>(op->max_local, op->max_for, op->max_own, own, halo)
+                     : patch_smem_bytes<K, T, 1>(op->max_local, op->max_for, op->max_own, own, halo);
 }
 
 constexpr size_t kSmemLimit = 227 * 1024;
@@ -555,100 +559,101 @@ void with_kernels(const geo_op* op, F&& f) {
     }
 }
 
-template <class K, class T, int NBUF>
-int setup_patch_nbuf(size_t attr_bytes, size_t plain, size_t own, int& per_sm_plain) {
-    GEO_CUDA(cudaFuncSetAttribute(k_patch<K, T, MODE_FREE, NBUF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)attr_bytes));
-    GEO_CUDA(cudaFuncSetAttribute(k_patch<K, T, MODE_LIFT, NBUF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)attr_bytes));
-    GEO_CUDA(cudaFuncSetAttribute(k_patch<K, T, MODE_PCG, NBUF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)attr_bytes));
-    GEO_CUDA(cudaFuncSetAttribute(k_patch<K, T, MODE_PCG, NBUF, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)attr_bytes));
-    GEO_CUDA(cudaFuncSetAttribute(k_patch<K, T, MODE_FREE, NBUF, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)attr_bytes));
-    GEO_CUDA(cudaFuncSetAttribute(k_patch<K, T, MODE_LIFT, NBUF, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)attr_bytes));
-    per_sm_plain = 0;
-    GEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_plain, k_patch<K, T, MODE_PCG, NBUF>, kPatchBS,
-                                                           plain));
-    int per_sm_own = 0;
-    if (own)
-        GEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_own, k_patch<K, T, MODE_PCG, NBUF>,
-                                                               kPatchBS, own));
-    return per_sm_own;
+// Calls f(kernel) for the patch kernel of one mode, buffer count and halo mode.
+template <class K, class T, int MODE, class F>
+void with_patch_kernel(int nbuf, int halo, F&& f) {
+    if (nbuf == 2) {
+        if (halo == 2) f(k_patch<K, T, MODE, 2, 2>);
+        else if (halo == 1) f(k_patch<K, T, MODE, 2, 1>);
+        else f(k_patch<K, T, MODE, 2, 0>);
+    } else {
+        if (halo == 2) f(k_patch<K, T, MODE, 1, 2>);
+        else if (halo == 1) f(k_patch<K, T, MODE, 1, 1>);
+        else f(k_patch<K, T, MODE, 1, 0>);
+    }
 }
 
-// Picks double buffering when it fits in shared memory, and the own-node bulk copies
-// (FP32 thermal PCG) when they cost no resident block: the gather then reads the
-// patch's own-node D^-1, r and p_old from shared memory, but their buffer (about 13
-// bytes per own node) took one block per SM away on meshes whose patches hold more
-// nodes, which was slower than the plain gather (80^3, 112^3). Returns the grid.
+// Lets a kernel take `bytes` of dynamic shared memory. The attribute belongs to the
+// kernel, not to the operator, so it is only ever raised: a smaller operator made later
+// must not take it from a larger one that is still in use.
+template <class Kernel>
+void allow_smem(Kernel k, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, size_t> allowed;
+    int dev = 0;
+    GEO_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& a = allowed[{dev, (const void*)k}];
+    if (bytes <= a) return;
+    GEO_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    a = bytes;
+}
+
+// Resident blocks per SM of the PCG-mode patch kernel.
+template <class K, class T>
+int patch_residency(int nbuf, int halo, size_t smem) {
+    int per_sm = 0;
+    if (smem > kSmemLimit) return 0;
+    with_patch_kernel<K, T, MODE_PCG>(nbuf, halo, [&](auto k) {
+        allow_smem(k, smem);
+        GEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kPatchBS, smem));
+    });
+    return per_sm;
+}
+
+// Chooses the form of the patch kernel, from its resident blocks per SM:
+// - two element-data buffers when they fit in shared memory, else one;
+// - halo mode when the operator has slots, the slot list in the bulk copy when that
+//   costs no resident block, else read by the flush from global memory;
+// - own-node slices by bulk copy (PCG) when their buffer costs no resident block:
+//   about 13 bytes per own node took one block per SM away on meshes whose patches hold
+//   more nodes, which was slower than the plain gather (80^3, 112^3).
+// GEO_PATCH_NBUF=1 and GEO_PATCH_HALO (0: atomics, 1: slots in shared memory, 2: slots
+// from global) force a form, so that tests cover all of them on small meshes. Returns
+// the grid.
 template <class K, class T>
 int setup_patch_kernels(geo_op* op, int slot) {
-    int nbuf = 2;
-    // GEO_PATCH_NBUF=1 forces the single-buffer kernel, so that tests cover it on small meshes
     const char* force_nbuf = std::getenv("GEO_PATCH_NBUF");
-    if (smem_bytes<K, T>(op, 2, false) > kSmemLimit || (force_nbuf && std::strcmp(force_nbuf, "1") == 0)) {
-        if (smem_bytes<K, T>(op, 1, false) > kSmemLimit)
-            fail(GEO_ERR_UNSUPPORTED, "patch tables exceed shared memory (too many nodes per patch)");
-        nbuf = 1;
-    }
-    op->nbuf[slot] = nbuf;
-    const size_t plain = smem_bytes<K, T>(op, nbuf, false);
-    size_t own = own_bulk<K, T, MODE_PCG>() ? smem_bytes<K, T>(op, nbuf, true) : 0;
-    if (own > kSmemLimit) own = 0;
-    int per_sm = 0;
-    const int per_sm_own = nbuf == 2 ? setup_patch_nbuf<K, T, 2>(std::max(plain, own), plain, own, per_sm)
-                                     : setup_patch_nbuf<K, T, 1>(std::max(plain, own), plain, own, per_sm);
-    op->own_bulk[slot] = own && per_sm_own >= per_sm;
-    op->patch_smem[slot] = op->own_bulk[slot] ? own : plain;
-    if (per_sm < 1) fail(GEO_ERR_UNSUPPORTED, "patch kernel does not fit on an SM");
-    per_sm = std::max(per_sm, per_sm_own);
-    // halo mode: slots in the bulk copy when that costs no
-    // resident block, else read by the flush from global memory. GEO_PATCH_HALO
-    // (0: atomics, 1: slots in shared memory, 2: slots from global) forces a mode,
-    // so that tests cover all three on small meshes.
-    op->halo[slot] = 0;
     const char* force = std::getenv("GEO_PATCH_HALO");
     const int forced = force && force[0] >= '0' && force[0] <= '2' && force[1] == 0 ? force[0] - '0' : -1;
-    if ((K::DPN == 1 || K::DPN == 3) && op->halo_ok && forced != 0) {
-        op->halo[slot] = 2;
-        const size_t hs = smem_bytes<K, T>(op, nbuf, op->own_bulk[slot] != 0, 1);
-        int per_sm_halo = 0;
-        if (hs <= kSmemLimit) {  // raises the limit of every mode (all launch with patch_smem[slot])
-            const size_t attr = std::max(hs, std::max(plain, own));
-            if (nbuf == 2) setup_patch_nbuf<K, T, 2>(attr, hs, 0, per_sm_halo);
-            else setup_patch_nbuf<K, T, 1>(attr, hs, 0, per_sm_halo);
-        }
-        if (per_sm_halo > 0 && (forced == 1 || (forced < 0 && per_sm_halo >= per_sm))) {
-            op->halo[slot] = 1;
-            op->patch_smem[slot] = hs;
-            if (forced == 1) per_sm = per_sm_halo;
-        }
-        if (forced == 2) {
-            op->halo[slot] = 2;
-            op->patch_smem[slot] = op->own_bulk[slot] ? own : plain;
+    const bool halo_ok = op->halo_ok && forced != 0;
+    int halo = halo_ok ? 2 : 0;
+    int nbuf = 2;
+    if (smem_bytes<K, T>(op, 2, false, halo) > kSmemLimit || (force_nbuf && std::strcmp(force_nbuf, "1") == 0)) nbuf = 1;
+    int per_sm = patch_residency<K, T>(nbuf, halo, smem_bytes<K, T>(op, nbuf, false, halo));
+    if (per_sm < 1) fail(GEO_ERR_UNSUPPORTED, "patch tables exceed shared memory (too many nodes per patch)");
+    bool own = false;
+    if (const int with_own = patch_residency<K, T>(nbuf, halo, smem_bytes<K, T>(op, nbuf, true, halo)); with_own >= per_sm) {
+        own = true;
+        per_sm = with_own;
+    }
+    if (halo_ok && forced != 2) {
+        const int in_copy = patch_residency<K, T>(nbuf, 1, smem_bytes<K, T>(op, nbuf, own, 1));
+        if (in_copy > 0 && (forced == 1 || in_copy >= per_sm)) {
+            halo = 1;
+            per_sm = in_copy;
         }
     }
+    op->nbuf[slot] = nbuf;
+    op->own_bulk[slot] = own;
+    op->halo[slot] = halo;
+    op->patch_smem[slot] = smem_bytes<K, T>(op, nbuf, own, halo);
+    // MODE_FREE and MODE_LIFT launch with the same shared memory
+    with_patch_kernel<K, T, MODE_FREE>(nbuf, halo, [&](auto k) { allow_smem(k, op->patch_smem[slot]); });
+    with_patch_kernel<K, T, MODE_LIFT>(nbuf, halo, [&](auto k) { allow_smem(k, op->patch_smem[slot]); });
     return per_sm * op->ctx->sm_count;
 }
 
+// Blocks of the patch kernel: the resident ones, or one per patch.
+unsigned patch_blocks(const geo_op* op, int slot) { return (unsigned)std::min(op->patch_grid[slot], op->n_patches); }
+
 template <class K, class T, int MODE>
 void launch_patch(const geo_op* op, int slot, cudaStream_t s, const T* qd, const PatchArgs<T>& pa) {
-    const unsigned g = (unsigned)std::min(op->patch_grid[slot], op->n_patches);
     PatchView v = view(op);
     v.own_bulk = op->own_bulk[slot];
-    v.halo = pa.halo ? op->halo[slot] : 0;  // halo mode whenever the caller passes the slot array
-    const size_t smem = op->patch_smem[slot];
-    const bool hg = v.halo == 2;
-    if (op->nbuf[slot] == 2) {
-        if (hg) k_patch<K, T, MODE, 2, 1><<<g, kPatchBS, smem, s>>>(v, qd, (T)op->cl, (T)op->cm, pa);
-        else k_patch<K, T, MODE, 2><<<g, kPatchBS, smem, s>>>(v, qd, (T)op->cl, (T)op->cm, pa);
-    } else {
-        if (hg) k_patch<K, T, MODE, 1, 1><<<g, kPatchBS, smem, s>>>(v, qd, (T)op->cl, (T)op->cm, pa);
-        else k_patch<K, T, MODE, 1><<<g, kPatchBS, smem, s>>>(v, qd, (T)op->cl, (T)op->cm, pa);
-    }
+    with_patch_kernel<K, T, MODE>(op->nbuf[slot], op->halo[slot], [&](auto k) {
+        k<<<patch_blocks(op, slot), kPatchBS, op->patch_smem[slot], s>>>(v, qd, (T)op->cl, (T)op->cm, pa);
+    });
 }
 
 // Halo slots (see k_halo_count): fslot in the fids
@@ -760,10 +765,8 @@ void refresh_coefficients(geo_op* op) {
     double maxd;
     std::memcpy(&maxd, &bits, sizeof(double));
     op->cd = maxd > 1.0 ? maxd : 1.0;  // assembly.rs:184-193
-    // padded to whole 64-entry blocks: the patch kernel copies ranges rounded outwards to 16 bytes
-    op->dinv64.ensure((size_t)(op->ndof + 63) / 64 * 64);
-    // padded to whole 64-entry blocks: the patch kernel copies ranges rounded outwards to 4 values
-    op->dinv32.ensure((size_t)(op->ndof + 63) / 64 * 64);
+    op->dinv64.ensure(padded_dofs(op));
+    op->dinv32.ensure(padded_dofs(op));
     op->diag_new.ensure(op->ndof);
     k_dinv<<<nblk(op->ndof), 256, 0, s>>>(op->nperm.p, op->flags.p, op->dpn, op->N, op->diag_orig.p, op->cd,
                                          op->dinv64.p, op->dinv32.p, op->diag_new.p);
@@ -816,6 +819,7 @@ geo_op* create_op(geo_ctx* ctx, const geo_mesh* mesh, const geo_dofs* dofs, int 
     op->pf = std::move(L.patch_foreign);
     op->foreign = std::move(L.foreign);
     op->lc = std::move(L.lc);
+    op->lc32 = std::move(L.lc32);
     op->mask_orig.alloc(op->ndof);
     GEO_CUDA(cudaMemcpyAsync(op->mask_orig.p, dofs->mask.p, op->ndof, cudaMemcpyDeviceToDevice, s));
     // padded to 16 bytes: the patch kernel copies flag ranges rounded outwards to 16
@@ -895,9 +899,10 @@ geo_op* create_op(geo_ctx* ctx, const geo_mesh* mesh, const geo_dofs* dofs, int 
     });
     op->bvec.alloc(op->ndof);
     op->xvec.alloc(op->ndof);
-    op->state.alloc(1);
-    op->part.alloc((size_t)2 * std::max({op->patch_grid[0], op->patch_grid[1], op->node_grid[0], op->node_grid[1]}));
-    GEO_CUDA(cudaMemset(op->state.p, 0, sizeof(PcgState)));
+    op->state.alloc(2);
+    op->part.alloc((size_t)2 * std::max(op->node_grid[0], op->node_grid[1]));
+    op->part_patch.alloc((size_t)2 * std::max(op->patch_grid[0], op->patch_grid[1]));
+    GEO_CUDA(cudaMemset(op->state.p, 0, op->state.bytes()));
     GEO_CUDA(cudaMallocHost(&op->h_state, sizeof(PcgState)));
     return op.release();
 }
@@ -959,12 +964,26 @@ void lift_new(geo_op* op, const double* f_orig_dev, double* fbc_new) {
     sync(op->ctx, "lift");
 }
 
+// Blocks of a node kernel whose threads take `items` items: one wave of resident
+// blocks, or as many as there is work for. Every block costs a ticket and a partial in
+// the last block's sum.
+unsigned node_blocks(const geo_op* op, int slot, int64_t items) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(op->node_grid[slot], cdiv(items, kNodeBS)));
+}
+
+// Blocks of the node update. Its items: a 16-byte vector (one DOF per node; the atomics
+// form), else one node (FP64) or two (FP32) of the three-DOF halo form.
+unsigned update_blocks(const geo_op* op, int slot) {
+    return node_blocks(op, slot, op->dpn == 1 || !op->halo[slot] ? cdiv(op->ndof, slot ? 4 : 2)
+                                                                 : (slot ? cdiv(op->N, 2) : op->N));
+}
+
 // The node update of the PCG loop: the halo-mode kernel when the patch kernel runs
 // in halo mode.
 template <class K, class T, bool MIXED>
 void launch_update(const geo_op* op, cudaStream_t s, const NodeArgs<T>& na) {
     constexpr int slot = std::is_same<T, double>::value ? 0 : 1;
-    const unsigned g = (unsigned)op->node_grid[slot];
+    const unsigned g = update_blocks(op, slot);
     if (op->halo[slot]) k_pcg_update_halo<T, K::DPN, MIXED><<<g, kNodeBS, 0, s>>>(na);
     else k_pcg_update<T, K::DPN, MIXED><<<g, kNodeBS, 0, s>>>(na);
 }
@@ -991,7 +1010,7 @@ PcgLaunchArgs pcg_args(geo_op* op, bool mixed) {
     const int64_t n = op->ndof;
     // sub-arrays at a common stride of whole 256-byte blocks, so that all vectors of
     // the node update share 16-byte alignment
-    const int64_t np = (n + 63) / 64 * 64;
+    const int64_t np = (int64_t)padded_dofs(op);
     op->w64.ensure((size_t)(mixed ? 1 : 4) * np);
     if (mixed) op->w32.ensure((size_t)5 * np);
     PcgLaunchArgs a;
@@ -1002,10 +1021,21 @@ PcgLaunchArgs pcg_args(geo_op* op, bool mixed) {
     n64.flags = n32.flags = op->flags.p;
     n64.n = n32.n = n;
     n64.dpn = n32.dpn = op->dpn;
-    n64.st = n32.st = p64.st = p32.st = op->state.p;
+    // the patch kernel reads the first copy of the state and writes the second, the
+    // node update the other way round; each kernel folds the other's partials in
+    n64.st = n32.st = op->state.p;
+    n64.st_in = n32.st_in = op->state.p + 1;
+    p64.st = p32.st = op->state.p;
+    p64.st_out = p32.st_out = op->state.p + 1;
     p64.err = p32.err = &op->state.p->err;
     n64.part = n32.part = op->part.p;
-    p64.part = p32.part = op->part.p;  // patch and node kernels never overlap
+    p64.part_in = p32.part_in = op->part.p;
+    p64.part = p32.part = op->part_patch.p;
+    n64.part_in = n32.part_in = op->part_patch.p;
+    p64.n_in = (int)update_blocks(op, 0);
+    p32.n_in = (int)update_blocks(op, 1);
+    n64.n_in = (int)patch_blocks(op, 0);
+    n32.n_in = (int)patch_blocks(op, 1);
     n64.b = n32.b = op->bvec.p;
     n64.x64 = n32.x64 = op->xvec.p;
     if (!mixed) {
@@ -1045,9 +1075,6 @@ PcgLaunchArgs pcg_args(geo_op* op, bool mixed) {
         n32.halo = p32.halo = op->halo32.p;
         n32.hbase = op->hbase.p;
     }
-    auto al = [](const void* q) { return ((uintptr_t)q & 15u) == 0; };
-    n64.vec = al(n64.x) && al(n64.r) && al(n64.q) && al(n64.dinv) && al(n64.pbuf0) && al(n64.pbuf1);
-    n32.vec = al(n32.x) && al(n32.r) && al(n32.q) && al(n32.dinv) && al(n32.pbuf0) && al(n32.pbuf1);
     return a;
 }
 
@@ -1055,7 +1082,7 @@ PcgLaunchArgs pcg_args(geo_op* op, bool mixed) {
 void pcg_start(geo_op* op, bool mixed, const PcgState& init, const PcgLaunchArgs& a) {
     cudaStream_t s = op->ctx->stream;
     GEO_CUDA(cudaMemcpyAsync(op->state.p, &init, sizeof(init), cudaMemcpyHostToDevice, s));
-    const unsigned ng = (unsigned)op->node_grid[mixed ? 1 : 0];
+    const unsigned ng = node_blocks(op, mixed ? 1 : 0, op->ndof);
     if (mixed) {
         k_mixed_init1<<<ng, kNodeBS, 0, s>>>(a.n32);
         k_mixed_init2<<<ng, kNodeBS, 0, s>>>(a.n32);
@@ -1086,7 +1113,7 @@ int solve_new(geo_op* op, const geo_cg_opts& o, geo_solver_stats* st) {
     const PatchArgs<double>& p64 = la.p64;
     const PatchArgs<float>& p32 = la.p32;
     const NodeArgs<double>& n64 = la.n64;
-    const unsigned ng = (unsigned)op->node_grid[mixed ? 1 : 0];
+    const unsigned ng = node_blocks(op, mixed ? 1 : 0, op->ndof);
     GEO_CUDA(cudaEventRecord(ctx->ev0, s));
     pcg_start(op, mixed, init, la);
     // (re)build the chunk graph when the buffers it captured changed
@@ -1104,6 +1131,8 @@ int solve_new(geo_op* op, const geo_cg_opts& o, geo_solver_stats* st) {
                 else enqueue_iteration<decltype(k64), double, false>(op, s, p64, n64);
             }
         });
+        if (mixed) k_pcg_decide<true><<<1, kNodeBS, 0, s>>>(op->state.p, p32.part_in, p32.n_in);
+        else k_pcg_decide<false><<<1, kNodeBS, 0, s>>>(op->state.p, p64.part_in, p64.n_in);
         GEO_CUDA(cudaStreamEndCapture(s, &g));
         GEO_CUDA(cudaGraphInstantiate(&op->chunk[pi], g, 0));
         cudaGraphDestroy(g);
@@ -1114,7 +1143,7 @@ int solve_new(geo_op* op, const geo_cg_opts& o, geo_solver_stats* st) {
     const long long max_rounds = o.max_iterations / 1 + 64;
     for (long long round = 0; round <= max_rounds; ++round) {
         GEO_CUDA(cudaGraphLaunch(op->chunk[pi], s));
-        launches += 2 * kChunk;
+        launches += 2 * kChunk + 1;
         GEO_CUDA(cudaMemcpyAsync(op->h_state, op->state.p, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
         sync(ctx, "PCG chunk");
         if (op->h_state->err) fail(GEO_ERR_TIMEOUT, "matrix-free PCG: a bounded device-side wait timed out");

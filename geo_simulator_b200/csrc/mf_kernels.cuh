@@ -8,7 +8,8 @@
 // next patch's copy is in flight while the current one is processed; the gather
 // then needs a single round trip to global memory. Per patch:
 //   1. gather: every patch-local node's input value is read once from global
-//      memory into a shared table (own nodes form one contiguous range);
+//      memory into a shared table (own nodes form one contiguous range, worked on in
+//      aligned groups with 16-byte accesses);
 //   2. element pass: each thread applies K_e to its elements from the shared
 //      table and accumulates into a shared output table with shared atomics
 //      (exact INT32 fixed point for FP32, see Scatter). Elements are ordered so
@@ -29,10 +30,18 @@
 // q = char_diag p), z = D^-1 r, and the r.r / r.z partial sums; loads are
 // issued for several entries before any store so they overlap.
 //
-// Every reduction is single pass: each block writes its partial, the last block
-// to finish (ticket counter) sums the partials in a fixed order and updates the
-// device-resident PcgState, which the next kernel reads. No host round trip per
-// iteration and no grid-wide spin wait.
+// Reductions of the PCG loop: each block of a kernel writes its partial sums, and
+// every block of the next kernel adds all of them in the same fixed order at its
+// start, while its first loads are in flight, and derives the iteration's scalars
+// from the totals (pcg_fold_update, pcg_fold_patch); block 0 stores them. A last-block
+// sum at the end of each kernel instead (fence, ticket, one warp walking the partials,
+// scalars, state store, then the next kernel's load of the state) put 3 to 4 us of
+// dependent latency behind each of the two kernels: with the folds an iteration takes
+// 13.0 instead of 19.0 us at 6^3 (FP64), 23.9 instead of 33.4 us at 48x48x32 (mixed)
+// and 24.1 instead of 31.0 us for FP64 elasticity at 27x22x13. Two copies of PcgState alternate, so that block 0 never
+// writes the copy that other blocks of its grid still read. The kernels outside the
+// loop (start, refresh) keep the ticket form. No host round trip per iteration and
+// no grid-wide spin wait.
 #pragma once
 
 #include <type_traits>
@@ -45,11 +54,10 @@ namespace geo {
 constexpr int kPatchBS = 192;  // threads of the patch kernel (2 elements each)
 constexpr int kNodeBS = 256;   // threads of the node kernels
 constexpr int kUnroll = 4;     // entries in flight per thread in the node kernels
-constexpr int kGather = 4;     // patch-local nodes in flight per thread in the gather
+constexpr int kForeignFlight = 2;  // foreign nodes in flight per thread in the gather
 
 enum : int { MODE_FREE = 0, MODE_LIFT = 1, MODE_PCG = 2 };
 enum : int { ST_DONE = 1, ST_REFRESH = 2, ST_CONVERGED = 4, ST_BREAKDOWN = 8 };
-enum : int { TICKET_PATCH = 0, TICKET_UPDATE = 1, TICKET_AUX = 2 };
 
 struct PatchMeta;
 
@@ -60,7 +68,8 @@ struct PatchView {
     const int32_t* po;
     const int32_t* pf;
     const int32_t* foreign;
-    const uint32_t* lc;  // patch-major paired connectivity [P][5][kPatchElems]
+    const uint32_t* lc;    // patch-major paired connectivity [P][5][kPatchElems], FP64 kernels
+    const uint32_t* lc32;  // the same for the FP32 kernels (PatchLayout::lc32)
     const uint8_t* flags;
     // scatter bound per patch (see Scatter): (max element incidences of a
     // patch-local node) x max_e ||K_e||_inf x 1.001, rounded up
@@ -74,12 +83,8 @@ struct PatchView {
     int max_for;
     int max_own;   // the largest own-node count of a patch
     int own_bulk;  // own-node slices by bulk copy (FP32 thermal PCG; the launch's shared memory holds them)
-    // halo mode (PCG): the halo slot of every foreign entry, in
-    // the same per-patch segments as fids. halo: 0 off; 1 the slots ride in the
-    // patch's bulk copy; 2 the flush reads them from global memory (coalesced), for
-    // launches where the shared-memory copy would cost a resident block
+    // halo mode: the halo slot of every foreign entry, in the same per-patch segments as fids
     const int32_t* fslot;
-    int halo;
     // per patch: element count, own range, foreign count and segment start, scatter
     // bound, as one 32-byte record (16-byte aligned), so that the patch kernel's
     // copy issue needs one prefetched record instead of dependent global loads
@@ -101,73 +106,114 @@ struct PatchView {
 // element incidences per node bounds the sum (PatchView::bound32).
 // FP32: one word (|sum| < 2^30, resolution 2^-30 of the bound). FP64: three
 // words holding hi 2^42 + mid 2^21 + lo (|sum| < 2^62, resolution 2^-62 of the
-// bound, below the FP64 rounding of the result). Word w of DOF slot s sits at
-// acc[w * m + s].
+// bound, below the FP64 rounding of the result).
 template <class T>
 struct Scatter;
 
 template <>
 struct Scatter<float> {
-    static constexpr float kLim = 1073741824.0f;  // 2^30
     static constexpr int kLimExp = 30;
     static constexpr int kWords = 1;
-    __device__ __forceinline__ static void zero(int* acc, int, int slot) { acc[slot] = 0; }
-    __device__ __forceinline__ static void add(int* acc, int, int slot, float v) {
-        atomicAdd(acc + slot, __float2int_rn(v));
-    }
-    __device__ __forceinline__ static float get(const int* acc, int, int slot) { return (float)acc[slot]; }
-    // read and clear (the flush leaves the table zero for the next patch)
-    __device__ __forceinline__ static float take(int* acc, int, int slot) {
-        const int v = acc[slot];
-        acc[slot] = 0;
-        return (float)v;
-    }
 };
 
 template <>
 struct Scatter<double> {
-    static constexpr float kLim = 4.611686018427388e18f;  // 2^62
     static constexpr int kLimExp = 62;
     static constexpr int kWords = 3;
-    __device__ __forceinline__ static void zero(int* acc, int m, int slot) {
-        acc[slot] = 0;
-        acc[m + slot] = 0;
-        acc[2 * m + slot] = 0;
+};
+
+// The patch-local node table: values x and fixed-point accumulators of every local
+// node, addressed by the node's handle, which comes from the element connectivity
+// (of_lc) or from the local index u (of_node; consecutive nodes of one aligned group
+// are kStep apart).
+template <class T, int DPN>
+struct NodeTable;
+
+// FP32: rows of 32 nodes, each row the nodes' values and then their accumulators, so
+// that both sit at fixed distances from one byte address (see patch_slot32).
+template <int DPN>
+struct NodeTable<float, DPN> {
+    unsigned char* tab;
+    __device__ NodeTable(unsigned char* base, int) : tab(base) {}
+    __host__ __device__ static size_t bytes(int max_local) { return (size_t)(max_local + 32) / 33 * (66 * 4 * DPN); }
+    static constexpr int kStep = 4 * DPN;
+    __device__ __forceinline__ static int of_lc(uint32_t v) { return (int)v * DPN; }
+    __device__ __forceinline__ static int of_node(int u) { return patch_slot32(u) * (4 * DPN); }
+    __device__ __forceinline__ float& x(int h, int c) const { return *reinterpret_cast<float*>(tab + h + 4 * c); }
+    __device__ __forceinline__ int& acc(int h, int c) const {
+        return *reinterpret_cast<int*>(tab + 33 * 4 * DPN + h + 4 * c);
     }
+    __device__ __forceinline__ void add(int h, int c, float v) const { atomicAdd(&acc(h, c), __float2int_rn(v)); }
+    // read and clear (the flush leaves the table zero for the next patch)
+    __device__ __forceinline__ float take(int h, int c) const {
+        int& a = acc(h, c);
+        const int v = a;
+        a = 0;
+        return (float)v;
+    }
+};
+
+// FP64: the values by slot, then the three accumulator words, word w of slot s at w M + s.
+template <int DPN>
+struct NodeTable<double, DPN> {
+    double* xs;
+    int* ys;
+    int M;
+    __device__ NodeTable(unsigned char* base, int max_local)
+        : xs(reinterpret_cast<double*>(base)), ys(reinterpret_cast<int*>(base + (size_t)max_local * DPN * 8)),
+          M(max_local * DPN) {}
+    __host__ __device__ static size_t bytes(int max_local) { return (size_t)max_local * DPN * (8 + 3 * 4); }
+    static constexpr int kStep = DPN;
+    __device__ __forceinline__ static int of_lc(uint32_t v) { return (int)v * DPN; }
+    __device__ __forceinline__ static int of_node(int u) { return patch_slot(u) * DPN; }
+    __device__ __forceinline__ double& x(int h, int c) const { return xs[h + c]; }
     // v = hi 2^42 + mid 2^21 + lo; hi and mid are exact, lo rounds the last fraction
-    __device__ __forceinline__ static void add(int* acc, int m, int slot, double v) {
+    __device__ __forceinline__ void add(int h, int c, double v) const {
         const int hi = __double2int_rn(v * 2.2737367544323206e-13);  // 2^-42
         const double r = fma(-(double)hi, 4398046511104.0, v);         // 2^42, exact
         const int mid = __double2int_rn(r * 4.76837158203125e-07);    // 2^-21
         const int lo = __double2int_rn(fma(-(double)mid, 2097152.0, r));
-        atomicAdd(acc + slot, hi);
-        atomicAdd(acc + m + slot, mid);
-        atomicAdd(acc + 2 * m + slot, lo);
+        int* acc = ys + h + c;
+        atomicAdd(acc, hi);
+        atomicAdd(acc + M, mid);
+        atomicAdd(acc + 2 * M, lo);
     }
-    __device__ __forceinline__ static double get(const int* acc, int m, int slot) {
-        return fma((double)acc[slot], 4398046511104.0, fma((double)acc[m + slot], 2097152.0, (double)acc[2 * m + slot]));
-    }
-    __device__ __forceinline__ static double take(int* acc, int m, int slot) {
-        const double v = get(acc, m, slot);
-        zero(acc, m, slot);
+    __device__ __forceinline__ double take(int h, int c) const {
+        int* acc = ys + h + c;
+        const double v = fma((double)acc[0], 4398046511104.0, fma((double)acc[M], 2097152.0, (double)acc[2 * M]));
+        acc[0] = acc[M] = acc[2 * M] = 0;
         return v;
     }
 };
 
-// S = the largest power of two <= 2^lim_exp / bx, clamped to [2^-100, 2^100], and
+// S = the largest power of two <= 2^lim_exp / bx, clamped to [2^-100, 2^hi], and
 // 1/S, both exact, from the exponent field of bx > 0 (no division): with
 // bx = m 2^e, m in [1, 2), S = 2^(lim_exp - e) when m = 1, else 2^(lim_exp - e - 1);
 // a subnormal bx gives the upper clamp, an infinite one the lower.
-__device__ __forceinline__ void pow2_scale(float bx, int lim_exp, float& S, float& invS) {
+__device__ __forceinline__ void pow2_scale(float bx, int lim_exp, int hi, float& S, float& invS) {
     const unsigned bits = __float_as_uint(bx);
     const int ef = (int)(bits >> 23);
     int se = lim_exp - (ef - 127) - ((bits & 0x7fffffu) != 0u ? 1 : 0);
-    if (ef == 0) se = 100;
+    if (ef == 0) se = hi;
     if (ef == 255) se = -100;
-    se = min(max(se, -100), 100);
+    se = min(max(se, -100), hi);
     S = __uint_as_float((unsigned)(se + 127) << 23);
     invS = __uint_as_float((unsigned)(127 - se) << 23);
 }
+
+// 16-byte vector of T
+template <class T>
+struct Vec16;
+template <>
+struct Vec16<float> {
+    using type = float4;
+    static constexpr int N = 4;
+};
+template <>
+struct Vec16<double> {
+    using type = double2;
+    static constexpr int N = 2;
+};
 
 // float <-> unsigned key with the same order (for warp min/max reductions)
 __device__ __forceinline__ unsigned float_key(float f) {
@@ -179,13 +225,18 @@ __device__ __forceinline__ float key_float(unsigned k) {
 }
 
 // Device-resident PCG scalars.
-struct PcgState {
+struct PcgScalars {
     double rz, rz_old, pAp, alpha, beta, bnorm, s_scale, rmax, res, ratio, s_new;
     double tol, abs_tol, delta, cd;
     long long it, max_it, nupd;
     int flags;
-    int err;  // DEV_ERR_* bits raised by bounded waits
-    unsigned int ticket[4];
+    int pending;  // the node update's partials (r.r, r.z) are not folded in yet
+};
+// With the words that the kernels of the loop do not copy along: the DEV_ERR_* bits
+// raised by bounded waits and the ticket counter (first copy only).
+struct PcgState : PcgScalars {
+    int err;
+    unsigned int ticket;
 };
 
 template <class T>
@@ -197,8 +248,11 @@ struct PatchArgs {
     const T* dinv;
     T* pbuf0;
     T* pbuf1;
-    PcgState* st;
-    double* part;  // [gridDim.x][2]
+    const PcgState* st;    // state left by the node update (or the start / refresh kernels)
+    PcgState* st_out;      // the state the node update reads
+    const double* part_in; // [n_in][2] partials of the node update
+    int n_in;
+    double* part;          // [gridDim.x][2] p.Ap partials of this kernel
     int* err;      // DEV_ERR_* bits (bounded waits)
     T* halo;       // halo mode: foreign contributions by slot (DPN values each)
     T* xsol;       // PCG z-form: the FP32 solution correction, updated on the own nodes
@@ -243,15 +297,97 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     return true;
 }
 
-// Last-block detection after every block stored its partial.
+// Last-block detection after every block stored its partial. Thread 0 wrote the
+// partial (store_partial), so its fence alone orders it before the ticket; the
+// block's other stores are for the next kernel.
 __device__ __forceinline__ bool last_block(unsigned int* ticket) {
     __shared__ int s_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
     __syncthreads();
     if (s_last) __threadfence();
     return s_last != 0;
+}
+
+// The scalars of an iteration that the kernels of the loop work with.
+struct PcgHead {
+    double alpha, beta, cd;
+    int odd;  // parity of the iteration count
+    int flags;
+};
+
+// The state after a node update whose sums of r.r and r.z are rr and rz: the stopping
+// and refresh tests and beta (iterative.rs:95-110).
+template <bool MIXED>
+__device__ __forceinline__ void pcg_next_iteration(PcgScalars& s, double rr, double rz) {
+    s.pending = 0;
+    const double rn = sqrt(rr);
+    if (!MIXED) {
+        s.res = rn;
+        if (rn < s.tol * s.bnorm || rn < s.abs_tol) {  // iterative.rs:95
+            s.flags |= ST_DONE | ST_CONVERGED;
+            return;
+        }
+    }
+    s.beta = rz / s.rz;
+    s.rz_old = s.rz;
+    s.rz = rz;
+    s.it += 1;
+    if (MIXED) {
+        s.rmax = fmax(s.rmax, rn);
+        const double est = rn * s.s_scale;
+        if (est < s.tol * s.bnorm || est < s.abs_tol || rn < s.delta * s.rmax || s.it >= s.max_it)
+            s.flags |= ST_REFRESH;
+    } else if (s.it >= s.max_it) {
+        s.flags |= ST_DONE;
+    }
+}
+
+// The state after a patch kernel whose sums are t[0] = sum_e p_e.K_e p_e and t[1] =
+// p.p over Dirichlet rows: p.Ap, alpha, breakdown (iterative.rs:85).
+__device__ __forceinline__ void pcg_step_length(PcgScalars& s, double t0, double t1) {
+    if (s.flags & (ST_DONE | ST_REFRESH)) return;
+    const double pAp = t0 + s.cd * t1;
+    s.pAp = pAp;
+    if (fabs(pAp) < 1e-30) {
+        s.flags |= ST_DONE | ST_BREAKDOWN;
+        s.alpha = 0.0;  // no step: the z-form's pending x update adds nothing
+    } else {
+        s.alpha = s.rz / pAp;
+        s.pending = 1;
+    }
+}
+
+// Start of a kernel of the loop: adds the previous kernel's partials and advances the
+// state with step(scalars, t0, t1). Every thread gets the scalars, block 0 stores the
+// state for the next kernel.
+template <class Step>
+__device__ __forceinline__ PcgHead pcg_fold(const PcgState* in, PcgState* out,
+                                            const double* __restrict__ part, int n, Step&& step) {
+    __shared__ PcgScalars s_st;  // worked on in place: few registers are live here
+    constexpr int kWords = sizeof(PcgScalars) / 8;
+    static_assert(sizeof(PcgScalars) % 8 == 0 && kWords <= 32, "the state is copied as 8-byte words by one warp");
+    double* words = reinterpret_cast<double*>(&s_st);
+    if (threadIdx.x < kWords)
+        words[threadIdx.x] = __ldcg(reinterpret_cast<const double*>(static_cast<const PcgScalars*>(in)) + threadIdx.x);
+    double t[2];
+    grid_sum0<2>(part, n, t);  // its block barriers order s_st before the reads below
+    if (threadIdx.x == 0) step(s_st, t[0], t[1]);
+    __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x < kWords)
+        reinterpret_cast<double*>(static_cast<PcgScalars*>(out))[threadIdx.x] = words[threadIdx.x];
+    return PcgHead{s_st.alpha, s_st.beta, s_st.cd, (int)(s_st.it & 1), s_st.flags};
+}
+
+// End of a chunk of iterations: folds the last node update's partials in, so that the
+// host reads a decided state. One block.
+template <bool MIXED>
+__global__ void __launch_bounds__(kNodeBS) k_pcg_decide(PcgState* st, const double* __restrict__ part, int n) {
+    pcg_fold(st, st, part, n, [](PcgScalars& s, double t0, double t1) {
+        if (s.pending) pcg_next_iteration<MIXED>(s, t0, t1);
+    });
 }
 
 // bytes of one patch's element data (connectivity + qdata), 16-byte multiple
@@ -293,7 +429,7 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// per-buffer bytes of [meta | foreign ids | foreign flags | halo slots (halo == 1)]
+// per-buffer bytes of [meta | foreign ids | foreign flags | halo slots (halo mode 1)]
 __host__ __device__ inline uint32_t patch_aux_ids(int max_for) {
     return round16((uint32_t)((max_for + kForeignAlign - 1) / kForeignAlign * kForeignAlign) * 4u);
 }
@@ -305,51 +441,38 @@ __host__ __device__ inline uint32_t patch_aux_bytes(int max_for, int halo) {
            (halo == 1 ? patch_aux_ids(max_for) : 0u);
 }
 
-// Own-node slices (PCG mode): D^-1, r and p_old over the patch's own DOF range
-// [dpn o0, dpn o1) (components interleaved, so the range is contiguous) and the
-// flags of its own nodes, copied with cp.async.bulk from 16-byte aligned starts
-// (ranges rounded outwards to 16 bytes). Capacities: values per array, flag bytes.
+// Own-node slices (PCG mode): D^-1, r and p_old (z-form: z, p_old, x) over the patch's
+// own nodes [o0, o1), rounded outwards to kNodeAlign nodes (components interleaved, so
+// the range is contiguous and starts on 16 bytes), and the flags of its own nodes,
+// copied with cp.async.bulk. Capacities: values per array, flag bytes.
 template <class T>
 __host__ __device__ inline uint32_t own_cap(int max_own, int dpn) {
-    constexpr uint32_t V = 16 / sizeof(T);
-    return ((uint32_t)(max_own * dpn) + 2 * V + V - 1) & ~(V - 1);
+    return (uint32_t)((max_own + 3 * kNodeAlign - 1) / kNodeAlign * kNodeAlign * dpn);
 }
 __host__ __device__ inline uint32_t own_capf(int max_own) { return (uint32_t)(max_own + 32 + 15) & ~15u; }
 template <class T>
 __host__ __device__ inline uint32_t own_bytes(int max_own, int dpn) {
     return 3u * own_cap<T>(max_own, dpn) * (uint32_t)sizeof(T) + own_capf(max_own);
 }
-template <class K, class T, int MODE>
-__host__ __device__ constexpr bool own_bulk() {
-    return MODE == MODE_PCG;
-}
 
-// Loop shape of the double-buffered patch kernel.
-// - Early (FP32 thermal): the next patch's copy is issued at the top of the loop,
-//   a whole patch ahead, and a block barrier after the flush frees the buffer it
-//   overwrites. Its gather is short next to the copy's latency.
-// - Late (the others): the copy is issued after the gather barrier, when every warp
-//   has left the previous flush. No barrier follows the flush, so fast warps start
-//   the next gather while others still flush; the node flags then need one table
-//   per patch parity.
+// shared memory layout: [3 mbarriers (32 B) | node table | NBUF x (lc | qd) | NBUF x (meta | foreign ids |
+// foreign flags | slots) | node flags (atomics mode) | own-node slices (PCG)]
+constexpr uint32_t kPatchBars = 32;
+template <class K, class T>
+__host__ __device__ inline uint32_t patch_table_bytes(int max_local) {
+    return round16((uint32_t)NodeTable<T, K::DPN>::bytes(max_local));
+}
+template <class K, class T>
+__host__ __device__ constexpr uint32_t patch_elem_bytes() { return patch_bytes_lc<K, T>() + patch_bytes_qd<K, T>(); }
 template <class K, class T, int NBUF>
-__host__ __device__ constexpr bool patch_late() {
-    return NBUF == 2 && !(K::DPN == 1 && sizeof(T) == 4);
+__host__ __device__ inline uint32_t patch_flag_bytes(int max_local, int halo) {
+    return halo ? 0u : round16((uint32_t)(max_local * NBUF));
 }
 template <class K, class T, int NBUF>
-__host__ __device__ constexpr int patch_flag_tables() {
-    return patch_late<K, T, NBUF>() ? 2 : 1;
-}
-
-// shared memory layout: [3 mbarriers (32 B) | NBUF x (lc | qd) | NBUF x (meta | foreign ids | foreign flags) |
-// xs | ys | flags (one table, two in the late shape) | own-node slices (PCG)]
-template <class K, class T, int NBUF>
-__host__ __device__ constexpr size_t patch_smem_fixed() {
-    return 32 + (size_t)NBUF * (patch_bytes_lc<K, T>() + patch_bytes_qd<K, T>());
-}
-template <class K, class T, int NBUF>
-__host__ __device__ inline size_t patch_smem_tables(int max_for, int halo) {
-    return patch_smem_fixed<K, T, NBUF>() + (size_t)NBUF * patch_aux_bytes(max_for, halo);
+__host__ __device__ inline size_t patch_smem_bytes(int max_local, int max_for, int max_own, bool own, int halo) {
+    return kPatchBars + patch_table_bytes<K, T>(max_local) + NBUF * patch_elem_bytes<K, T>() +
+           NBUF * patch_aux_bytes(max_for, halo) + patch_flag_bytes<K, T, NBUF>(max_local, halo) +
+           (own ? own_bytes<T>(max_own, K::DPN) : 0u);
 }
 
 // Resident blocks per SM the register allocation must allow (the minimum-blocks
@@ -362,38 +485,44 @@ __host__ __device__ constexpr int patch_min_blocks() {
     return sizeof(T) == 4 ? (K::DPN == 1 ? 0 : 2) : (K::DPN == 1 ? 2 : 1);
 }
 
-// HG = 1: the halo-mode variant whose flush reads the halo slots from global
-// memory (PatchView::halo == 2); HG = 0 serves every other launch.
-template <class K, class T, int MODE, int NBUF, int HG = 0>
+// HM: 0 atomics, 1 halo mode with the slots in the bulk copy, 2 halo mode with the slots
+// read from global memory by the flush.
+//
+// A patch's own nodes are gathered and flushed in aligned groups of V consecutive nodes
+// (16 bytes per component array) by one thread, with 16-byte accesses; only the edge
+// groups, which hold a neighbour patch's nodes too, go node by node. With the groups,
+// the foreign values requested before the flush of the patch before, one copy schedule
+// (late) for all kernels and the shorter affine apply, launches went from 264 to 249 us
+// (FP32 thermal, 128^3), 83 to 75 us (FP64 thermal, 64^3) and 37.3 to 33.2 us (FP32
+// elasticity, 48x48x24), events around each launch. The FP32 thermal kernel is bound by
+// the shared-memory pipe (67% of its wavefronts' peak, 4.4 per scatter atomic) and, at
+// 128^3, by the card's 1 kW power cap (clocks at 1.91 GHz); FP64 by latency (two blocks
+// of six warps per SM, issue 40%).
+template <class K, class T, int MODE, int NBUF, int HM>
 __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
     k_patch(PatchView pv, const T* __restrict__ qd_all, T cl, T cm, PatchArgs<T> a) {
     constexpr int DPN = K::DPN;
     constexpr uint32_t LCB = patch_bytes_lc<K, T>(), QDB = patch_bytes_qd<K, T>();
+    constexpr bool HALO = HM != 0;
+    using VT = typename Vec16<T>::type;
+    constexpr int V = Vec16<T>::N;  // nodes per group; DPN vectors of 16 bytes per array
+    using Table = NodeTable<T, DPN>;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem);  // [0..NBUF): element data; [2]: own-node slices
-    unsigned char* ebuf = smem + 32;
-    const bool OWNB = own_bulk<K, T, MODE>() && pv.own_bulk != 0;
-    using SC = Scatter<T>;
-    const int M = pv.max_local * DPN;  // DOF slots of the patch-local table (nodes by patch_slot)
-    unsigned char* abuf = smem + patch_smem_fixed<K, T, NBUF>();  // NBUF x (meta | ids | flags)
-    const bool HALO = HG != 0 || pv.halo != 0;
-    const int HMODE = !HALO ? 0 : (HG ? 2 : 1);  // 1: slots in shared memory, 2: from global
-    const uint32_t AUX = patch_aux_bytes(pv.max_for, HMODE), AIDS = patch_aux_ids(pv.max_for);
+    const bool OWNB = MODE == MODE_PCG && pv.own_bulk != 0;
+    const uint32_t AUX = patch_aux_bytes(pv.max_for, HM), AIDS = patch_aux_ids(pv.max_for);
     const uint32_t AFL = patch_aux_flags(pv.max_for);
-    T* xs = reinterpret_cast<T*>(smem + patch_smem_tables<K, T, NBUF>(pv.max_for, HMODE));
-    int* ys = reinterpret_cast<int*>(xs + M);  // fixed-point accumulators, SC::kWords x M words
+    const Table tab(smem + kPatchBars, pv.max_local);
+    unsigned char* ebuf = smem + kPatchBars + patch_table_bytes<K, T>(pv.max_local);
+    unsigned char* abuf = ebuf + NBUF * (LCB + QDB);  // NBUF x (meta | ids | flags | slots)
+    uint8_t* sfl0 = abuf + NBUF * AUX;                // node flags (atomics mode)
+    T* own_a = reinterpret_cast<T*>(sfl0 + patch_flag_bytes<K, T, NBUF>(pv.max_local, HM));
+    const uint32_t OCAP = own_cap<T>(pv.max_own, DPN);
+    T* own_b = own_a + OCAP;
+    T* own_c = own_b + OCAP;
+    uint8_t* own_f = reinterpret_cast<uint8_t*>(own_c + OCAP);
     // FP32 scatter: per component, min and max of x over the patch as order keys, by patch parity
     __shared__ unsigned s_lo[2][DPN], s_hi[2][DPN];
-    constexpr bool LATE = patch_late<K, T, NBUF>();
-    // node flags; in the late shape by patch parity, since the flush of one patch
-    // reads them while faster warps already gather the next one
-    uint8_t* sfl0 = reinterpret_cast<uint8_t*>(ys + SC::kWords * M);
-    const uint32_t OCAP = own_cap<T>(pv.max_own, DPN);
-    T* own_d = reinterpret_cast<T*>(
-        smem + (((size_t)(sfl0 + patch_flag_tables<K, T, NBUF>() * pv.max_local - smem) + 15) & ~(size_t)15));
-    T* own_r = own_d + OCAP;
-    T* own_p = own_r + OCAP;
-    uint8_t* own_f = reinterpret_cast<uint8_t*>(own_p + OCAP);
     // Preconditioned-residual form of the mixed solver's FP32 PCG (thermal and elasticity):
     // the node update keeps z = D^-1 r (a.r holds z) instead of r, so the gather
     // forms p = z + beta p_old from two vectors, and the solution update
@@ -405,13 +534,20 @@ __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
     const T* pold = nullptr;
     T* pnew = nullptr;
     if (MODE == MODE_PCG) {
-        if (a.st->flags & (ST_DONE | ST_REFRESH)) return;
-        beta = (T)a.st->beta;
-        if (ZF) alpha_prev = (T)a.st->alpha;
-        const bool odd = a.st->it & 1;
+        if (a.st->flags & (ST_DONE | ST_REFRESH)) {  // nothing to do, for the node update either
+            if (blockIdx.x == 0 && threadIdx.x == 0)
+                *static_cast<PcgScalars*>(a.st_out) = *static_cast<const PcgScalars*>(a.st);
+            return;
+        }
+        // the direction's buffer after the fold below: it counts the pending iteration
+        const bool odd = (a.st->it + a.st->pending) & 1;
         pold = odd ? a.pbuf1 : a.pbuf0;
         pnew = odd ? a.pbuf0 : a.pbuf1;
     }
+    // the three own-node arrays: z-form z, p_old, x; else D^-1, r, p_old
+    const T* ga = ZF ? a.r : a.dinv;
+    const T* gb = ZF ? pold : a.r;
+    const T* gc = ZF ? a.xsol : pold;
     if (threadIdx.x == 0) {
         for (int b = 0; b < NBUF; ++b) mbar_init(&bar[b], 1);
         if (OWNB) mbar_init(&bar[2], 1);
@@ -422,7 +558,8 @@ __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
         }
     }
     // the accumulators start at zero; each flush clears what it reads
-    for (int i = threadIdx.x; i < SC::kWords * M; i += blockDim.x) ys[i] = 0;
+    for (uint32_t i = threadIdx.x; i < patch_table_bytes<K, T>(pv.max_local) / 4; i += blockDim.x)
+        reinterpret_cast<int*>(smem + kPatchBars)[i] = 0;
     __syncthreads();
     // Thread 0 issues the copies of patch q_j (the block's j-th patch) from its record
     // in s_rec[j & 1], prefetched by cp.async when q_(j-1) was issued, so that no
@@ -435,32 +572,33 @@ __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
         cp_async_commit();
     };
     // thread 0: the patch's element data, sizes, foreign ids and foreign flags into buffer b
+    const uint32_t* lc_all = sizeof(T) == 4 ? pv.lc32 : pv.lc;
     auto issue = [&](const PatchMeta& m, int patch, int b) {
         unsigned char* ab = abuf + (size_t)b * AUX;
         *reinterpret_cast<PatchMeta*>(ab) = m;  // published by the arrive below
         const uint32_t ib = round16((uint32_t)m.nfor * 4u), fb = round16((uint32_t)m.nfor);
         unsigned char* dst = ebuf + (size_t)b * (LCB + QDB);
-        mbar_expect_tx(&bar[b], LCB + QDB + ib + fb + (HMODE == 1 ? ib : 0u));
-        bulk_g2s(dst, pv.lc + (size_t)patch * 5 * kPatchElems, LCB, &bar[b]);
+        mbar_expect_tx(&bar[b], LCB + QDB + ib + fb + (HM == 1 ? ib : 0u));
+        bulk_g2s(dst, lc_all + (size_t)patch * 5 * kPatchElems, LCB, &bar[b]);
         bulk_g2s(dst + LCB, qd_all + (size_t)patch * K::NQD * kPatchElems, QDB, &bar[b]);
         if (ib) {
             bulk_g2s(ab + sizeof(PatchMeta), pv.fids + m.fa, ib, &bar[b]);
             bulk_g2s(ab + sizeof(PatchMeta) + AIDS, pv.fflags + m.fa, fb, &bar[b]);
-            if (HMODE == 1) bulk_g2s(ab + sizeof(PatchMeta) + AIDS + AFL, pv.fslot + m.fa, ib, &bar[b]);
+            if (HM == 1) bulk_g2s(ab + sizeof(PatchMeta) + AIDS + AFL, pv.fslot + m.fa, ib, &bar[b]);
         }
     };
-    // thread 0: D^-1, r, p_old and flags of the patch's own nodes (single buffer, bar[2])
+    // thread 0: the own-node slices and flags of the patch's own nodes (single buffer, bar[2])
     auto issue_own = [&](const PatchMeta& m) {
-        constexpr int V = 16 / (int)sizeof(T);  // values per 16 bytes
         const int o0 = m.o0, o1 = m.o0 + m.nown;
-        const int a0 = (DPN * o0) & ~(V - 1), nv = ((DPN * o1 + V - 1) & ~(V - 1)) - a0;  // 16-byte aligned
-        const int f0 = o0 & ~15, nf = ((o1 + 15) & ~15) - f0;                             // flags, 16-byte aligned
-        const uint32_t vb = (uint32_t)nv * (uint32_t)sizeof(T);
+        const int n0 = patch_align(o0), nn = (o1 + kNodeAlign - 1) / kNodeAlign * kNodeAlign - n0;
+        const int f0 = o0 & ~15, nf = ((o1 + 15) & ~15) - f0;  // flags, 16-byte aligned
+        const uint32_t vb = (uint32_t)(nn * DPN) * (uint32_t)sizeof(T);
         mbar_expect_tx(&bar[2], 3u * vb + (uint32_t)nf);
-        if (nv) {  // z-form: z, p_old, x in the three slices; else D^-1, r, p_old
-            bulk_g2s(own_d, ZF ? a.r + a0 : a.dinv + a0, vb, &bar[2]);
-            bulk_g2s(own_r, ZF ? pold + a0 : a.r + a0, vb, &bar[2]);
-            bulk_g2s(own_p, ZF ? a.xsol + a0 : pold + a0, vb, &bar[2]);
+        if (vb) {
+            const int64_t at = (int64_t)n0 * DPN;
+            bulk_g2s(own_a, ga + at, vb, &bar[2]);
+            bulk_g2s(own_b, gb + at, vb, &bar[2]);
+            bulk_g2s(own_c, gc + at, vb, &bar[2]);
         }
         if (nf) bulk_g2s(own_f, pv.flags + f0, (uint32_t)nf, &bar[2]);
     };
@@ -481,23 +619,62 @@ __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
     uint32_t phase = 0;  // bit b = parity of buffer b; bit 2 = parity of the own-node buffer
     // bit b: a copy into buffer b is in flight (tracked by thread 0, which issues them)
     uint32_t pend = blockIdx.x < pv.n_patches ? (OWNB ? 5u : 1u) : 0u;
+    if (MODE == MODE_PCG) {  // the first patch's copies are in flight
+        const PcgHead h = pcg_fold(a.st, a.st_out, a.part_in, a.n_in, [](PcgScalars& s, double t0, double t1) {
+            if (s.pending) pcg_next_iteration<ZF>(s, t0, t1);
+        });
+        if (h.flags & (ST_DONE | ST_REFRESH)) {
+            if (threadIdx.x == 0) {  // let the copies land before the block's shared memory is released
+                for (int q = 0; q < 3; ++q)
+                    if ((pend >> q) & 1) mbar_wait(&bar[q], 0);
+                cp_async_wait_all();
+            }
+            return;
+        }
+        beta = (T)h.beta;
+        if (ZF) alpha_prev = (T)h.alpha;
+    }
+    // Foreign nodes go to scattered global addresses. Each thread has the values of up to
+    // kForeignFlight of them in flight: with two element buffers they are requested
+    // before the flush of the patch before (its element phase has brought the list), so
+    // that the flush and the own nodes of the gather cover their latency.
+    uint8_t ffl[kForeignFlight];
+    T f0[kForeignFlight][DPN], f1[kForeignFlight][DPN], f2[kForeignFlight][DPN];
+    auto f_load = [&](int b, int i, uint8_t& fl, T (&v0)[DPN], T (&v1)[DPN], T (&v2)[DPN]) {
+        const unsigned char* ab = abuf + (size_t)b * AUX;
+        if (i >= reinterpret_cast<const PatchMeta*>(ab)->nfor) return;
+        const int64_t at = (int64_t)reinterpret_cast<const int*>(ab + sizeof(PatchMeta))[i] * DPN;
+        fl = (ab + sizeof(PatchMeta) + AIDS)[i];
+#pragma unroll
+        for (int c = 0; c < DPN; ++c) {
+            if (MODE != MODE_PCG) {
+                v0[c] = a.x[at + c];
+            } else {
+                v0[c] = ga[at + c];
+                v1[c] = gb[at + c];
+                if (!ZF) v2[c] = gc[at + c];
+            }
+        }
+    };
+    // waits for the element data and lists in buffer b and requests the foreign values
+    auto arrive = [&](int b) {
+        if (!mbar_wait(&bar[b], (phase >> b) & 1)) return false;
+        phase ^= 1u << b;
+        pend &= ~(1u << b);
+#pragma unroll
+        for (int g = 0; g < kForeignFlight; ++g) f_load(b, threadIdx.x + g * kPatchBS, ffl[g], f0[g], f1[g], f2[g]);
+        return true;
+    };
     double dot = 0.0, pdd = 0.0;
+    // A thread whose bounded wait ran out skips the next gather, and the gather barrier
+    // ends the block.
+    bool ok = true;
+    if (NBUF == 2 && blockIdx.x < pv.n_patches) ok = arrive(0);
     int k = 0;
     for (int patch = blockIdx.x; patch < pv.n_patches; patch += gridDim.x, ++k) {
         const int b = NBUF == 2 ? (k & 1) : 0;
         const bool has_next = patch + (int)gridDim.x < pv.n_patches;
-        if (!LATE && NBUF == 2 && threadIdx.x == 0 && has_next) {
-            issue_next(patch, k, b ^ 1);
-            pend |= 1u << (b ^ 1);
-        }
-        // The patch's sizes, element data and foreign lists. No block barrier here: a
-        // thread whose bounded wait ran out skips the gather, and the gather barrier
-        // below ends the block.
-        bool ok = mbar_wait(&bar[b], (phase >> b) & 1);
-        if (ok) {
-            phase ^= 1u << b;
-            pend &= ~(1u << b);
-        }
+        if (NBUF == 1) ok = arrive(b);
         if (OWNB) {
             const bool ok2 = mbar_wait(&bar[2], (phase >> 2) & 1);
             if (ok2) {
@@ -506,99 +683,137 @@ __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
             }
             ok = ok && ok2;
         }
-        uint8_t* sfl = sfl0 + (LATE ? (k & 1) * pv.max_local : 0);
+        // node flags for the flush (atomics mode): with two buffers one table per patch
+        // parity, since the flush of one patch reads them while faster warps gather the next
+        uint8_t* sfl = sfl0 + b * pv.max_local;
         const unsigned char* ab = abuf + (size_t)b * AUX;
         const PatchMeta pm = *reinterpret_cast<const PatchMeta*>(ab);
         const int* __restrict__ sfor = reinterpret_cast<const int*>(ab + sizeof(PatchMeta));
-        const uint8_t* __restrict__ sffl = ab + sizeof(PatchMeta) + AIDS;
         const int* __restrict__ sfsl = reinterpret_cast<const int*>(ab + sizeof(PatchMeta) + AIDS + AFL);
-        const int n_el = pm.n_el, o0 = pm.o0, nown = pm.nown, nloc = nown + pm.nfor;
-        const float pbound = pm.bound;
+        const int o0 = pm.o0, o1 = pm.o0 + pm.nown, n0 = patch_align(o0);
+        const int uf = o1 - n0;  // local index of the first foreign node
         float xlo[DPN], xhi[DPN];
 #pragma unroll
         for (int c = 0; c < DPN; ++c) {
             xlo[c] = 3.0e38f;
             xhi[c] = -3.0e38f;
         }
-        // 1. gather (overlaps the bulk copies in flight); each thread issues the
-        //    loads of up to kGather nodes before any store
-        const int nloc_g = ok ? nloc : 0;
-        for (int u0 = threadIdx.x; u0 < nloc_g; u0 += kGather * blockDim.x) {
-            int node[kGather];
-            uint8_t fl[kGather];
-            T d0[kGather][DPN], d1[kGather][DPN], d2[kGather][DPN];
+        auto range = [&](int c, T v) {
+            xlo[c] = fminf(xlo[c], (float)v);
+            xhi[c] = fmaxf(xhi[c], (float)v);
+        };
+        // 1. gather
+        const int nfor = ok ? pm.nfor : 0, ngrp = ok ? (o1 - n0 + V - 1) / V : 0;
+        auto f_store = [&](int i, uint8_t fl, const T (&v0)[DPN], const T (&v1)[DPN], const T (&v2)[DPN]) {
+            if (i >= nfor) return;
+            const int h = Table::of_node(uf + i);
+            if (!HALO) sfl[uf + i] = fl;
 #pragma unroll
-            for (int g = 0; g < kGather; ++g) {
-                const int u = u0 + g * blockDim.x;
-                node[g] = u < nown ? o0 + u : (u < nloc ? sfor[u - nown] : 0);
+            for (int c = 0; c < DPN; ++c) {
+                const bool dir = (fl >> c) & 1;
+                T v;
+                if (MODE == MODE_PCG) v = dir ? T(0) : (ZF ? v0[c] + beta * v1[c] : v0[c] * v1[c] + beta * v2[c]);
+                else v = (MODE == MODE_FREE ? dir : !dir) ? T(0) : v0[c];
+                tab.x(h, c) = v;
+                range(c, v);
             }
+        };
+        for (int grp = threadIdx.x; grp < ngrp; grp += kPatchBS) {
+            const int j0 = n0 + V * grp;  // first node of the group
+            const bool full = j0 >= o0 && j0 + V <= o1;
+            const int64_t at = (int64_t)(j0 / V) * DPN;  // in vectors
+            VT va[DPN], vb[DPN], vc[DPN];
+            unsigned fw;
+            const uint8_t* fp = OWNB ? own_f + (j0 - (o0 & ~15)) : pv.flags + j0;
+            if (V == 4) fw = *reinterpret_cast<const uint32_t*>(fp);
+            else fw = *reinterpret_cast<const uint16_t*>(fp);
+            if (MODE != MODE_PCG) {
+                if (full) {
 #pragma unroll
-            for (int g = 0; g < kGather; ++g) {
-                const int u = u0 + g * blockDim.x;
-                if (OWNB && u < nown) {  // from the own-node slices in shared memory
-                    fl[g] = own_f[(o0 & 15) + u];
-                    const int base = ((DPN * o0) & (16 / (int)sizeof(T) - 1)) + DPN * u;
+                    for (int q = 0; q < DPN; ++q) va[q] = reinterpret_cast<const VT*>(a.x)[at + q];
+                } else {
 #pragma unroll
-                    for (int c = 0; c < DPN; ++c) {
-                        d0[g][c] = own_d[base + c];
-                        d1[g][c] = own_r[base + c];
-                        d2[g][c] = own_p[base + c];
+                    for (int e = 0; e < V; ++e)
+                        if (j0 + e >= o0 && j0 + e < o1)
+#pragma unroll
+                            for (int c = 0; c < DPN; ++c)
+                                reinterpret_cast<T*>(va)[e * DPN + c] = a.x[(int64_t)(j0 + e) * DPN + c];
+                }
+            } else if (OWNB) {
+#pragma unroll
+                for (int q = 0; q < DPN; ++q) {
+                    va[q] = reinterpret_cast<const VT*>(own_a)[grp * DPN + q];
+                    vb[q] = reinterpret_cast<const VT*>(own_b)[grp * DPN + q];
+                    vc[q] = reinterpret_cast<const VT*>(own_c)[grp * DPN + q];
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < DPN; ++q) {
+                    va[q] = reinterpret_cast<const VT*>(ga)[at + q];
+                    vb[q] = reinterpret_cast<const VT*>(gb)[at + q];
+                    vc[q] = reinterpret_cast<const VT*>(gc)[at + q];
+                }
+            }
+            T* ta = reinterpret_cast<T*>(va);  // becomes p (PCG)
+            const T* tb = reinterpret_cast<const T*>(vb);
+            T* tc = reinterpret_cast<T*>(vc);  // z-form: becomes x
+            const int h0 = Table::of_node(V * grp);
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                const bool in = full || (j0 + e >= o0 && j0 + e < o1);
+                if (!HALO && in) sfl[V * grp + e] = (uint8_t)(fw >> (8 * e));
+#pragma unroll
+                for (int c = 0; c < DPN; ++c) {
+                    const int q = e * DPN + c;
+                    const bool dir = (fw >> (8 * e + c)) & 1;
+                    T v;
+                    if (MODE == MODE_PCG) {
+                        const T pn = ZF ? ta[q] + beta * tb[q] : ta[q] * tb[q] + beta * tc[q];
+                        if (ZF) tc[q] = tc[q] + alpha_prev * tb[q];
+                        ta[q] = pn;
+                        if (dir && in) pdd += (double)(pn * pn);
+                        v = dir ? T(0) : pn;
+                    } else {
+                        v = (MODE == MODE_FREE ? dir : !dir) ? T(0) : ta[q];
                     }
-                } else if (u < nloc) {
-                    fl[g] = u < nown ? pv.flags[node[g]] : sffl[u - nown];
-#pragma unroll
-                    for (int c = 0; c < DPN; ++c) {
-                        const int64_t idx = (int64_t)node[g] * DPN + c;
-                        if (ZF) {
-                            d0[g][c] = a.r[idx];
-                            d1[g][c] = pold[idx];
-                            d2[g][c] = u < nown ? a.xsol[idx] : T(0);
-                        } else if (MODE == MODE_PCG) {
-                            d0[g][c] = a.dinv[idx];
-                            d1[g][c] = a.r[idx];
-                            d2[g][c] = pold[idx];
-                        } else {
-                            d0[g][c] = a.x[idx];
-                        }
+                    if (in) {
+                        tab.x(h0 + e * Table::kStep, c) = v;
+                        range(c, v);
                     }
                 }
             }
+            if (MODE == MODE_PCG) {
+                if (full) {
 #pragma unroll
-            for (int g = 0; g < kGather; ++g) {
-                const int u = u0 + g * blockDim.x;
-                if (u >= nloc) continue;
-                sfl[u] = fl[g];
-#pragma unroll
-                for (int c = 0; c < DPN; ++c) {
-                    const bool dir = (fl[g] >> c) & 1;
-                    T v;
-                    if (MODE == MODE_PCG) {
-                        const T pn = ZF ? d0[g][c] + beta * d1[g][c] : d0[g][c] * d1[g][c] + beta * d2[g][c];
-                        if (u < nown) {
-                            pnew[(int64_t)node[g] * DPN + c] = pn;
-                            if (ZF) a.xsol[(int64_t)node[g] * DPN + c] = d2[g][c] + alpha_prev * d1[g][c];
-                            if (dir) pdd += (double)(pn * pn);
-                        }
-                        v = dir ? T(0) : pn;
-                    } else {
-                        v = d0[g][c];
-                        if (MODE == MODE_FREE ? dir : !dir) v = T(0);
+                    for (int q = 0; q < DPN; ++q) {
+                        reinterpret_cast<VT*>(pnew)[at + q] = va[q];
+                        if (ZF) reinterpret_cast<VT*>(a.xsol)[at + q] = vc[q];
                     }
-                    xs[patch_slot(u) * DPN + c] = v;
-                    xlo[c] = fminf(xlo[c], (float)v);
-                    xhi[c] = fmaxf(xhi[c], (float)v);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < V; ++e)
+                        if (j0 + e >= o0 && j0 + e < o1)
+#pragma unroll
+                            for (int c = 0; c < DPN; ++c) {
+                                pnew[(int64_t)(j0 + e) * DPN + c] = ta[e * DPN + c];
+                                if (ZF) a.xsol[(int64_t)(j0 + e) * DPN + c] = tc[e * DPN + c];
+                            }
                 }
             }
         }
-        {
 #pragma unroll
-            for (int c = 0; c < DPN; ++c) {
-                const unsigned lo = __reduce_min_sync(0xffffffffu, float_key(xlo[c]));
-                const unsigned hi = __reduce_max_sync(0xffffffffu, float_key(xhi[c]));
-                if ((threadIdx.x & 31) == 0) {
-                    atomicMin(&s_lo[k & 1][c], lo);
-                    atomicMax(&s_hi[k & 1][c], hi);
-                }
+        for (int g = 0; g < kForeignFlight; ++g) f_store(threadIdx.x + g * kPatchBS, ffl[g], f0[g], f1[g], f2[g]);
+        for (int i = threadIdx.x + kForeignFlight * kPatchBS; i < nfor; i += kPatchBS) {
+            f_load(b, i, ffl[0], f0[0], f1[0], f2[0]);
+            f_store(i, ffl[0], f0[0], f1[0], f2[0]);
+        }
+#pragma unroll
+        for (int c = 0; c < DPN; ++c) {
+            const unsigned lo = __reduce_min_sync(0xffffffffu, float_key(xlo[c]));
+            const unsigned hi = __reduce_max_sync(0xffffffffu, float_key(xhi[c]));
+            if ((threadIdx.x & 31) == 0) {
+                atomicMin(&s_lo[k & 1][c], lo);
+                atomicMax(&s_hi[k & 1][c], hi);
             }
         }
         if (__syncthreads_or(!ok)) {
@@ -611,11 +826,11 @@ __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
             }
             return;
         }
-        // Every warp has left the previous patch's flush: in the late shape its buffer
+        // Every warp has left the previous patch's flush: with two buffers its buffer
         // takes the next patch's copy; the own-node buffer (read by the gather only)
         // takes the next patch's slices, during steps 2 and 3.
         if (threadIdx.x == 0 && has_next) {
-            if (LATE) {
+            if (NBUF == 2) {
                 issue_next(patch, k, b ^ 1);
                 pend |= 1u << (b ^ 1);
             }
@@ -640,10 +855,13 @@ __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
                     mabs = fmaxf(mabs, fmaxf(fabsf(lo), fabsf(hi)));
                 }
             }
-            const float bx = __fmul_ru(pbound, __fmaf_ru(mabs, 1.52587890625e-05f, half));  // 2^-16
+            const float bx = __fmul_ru(pm.bound, __fmaf_ru(mabs, 1.52587890625e-05f, half));  // 2^-16
             if (bx > 0.0f) {
+                // S multiplies G of the affine thermal elements (ThermalK::apply_affine): it
+                // stays below 2^120 / bound, and G below the bound on K_e's norm
+                const int cap = min(100, 246 - (int)(__float_as_uint(pm.bound) >> 23));
                 float sf, isf;
-                pow2_scale(bx, SC::kLimExp, sf, isf);
+                pow2_scale(bx, Scatter<T>::kLimExp, DPN == 1 && sizeof(T) == 4 ? cap : 100, sf, isf);
                 S = (T)sf;
                 invS = (T)isf;
             }
@@ -654,69 +872,85 @@ __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
         }
         const uint32_t* lcs = reinterpret_cast<const uint32_t*>(ebuf + (size_t)b * (LCB + QDB));
         const T* qds = reinterpret_cast<const T*>(ebuf + (size_t)b * (LCB + QDB) + LCB);
-        for (int el = threadIdx.x; el < n_el; el += blockDim.x) {
-            int li[10];
+        for (int el = threadIdx.x; el < pm.n_el; el += kPatchBS) {
+            int h[10];
             T xe[10 * DPN], ye[10 * DPN];
 #pragma unroll
             for (int l2 = 0; l2 < 5; ++l2) {
                 const uint32_t w = lcs[l2 * kPatchElems + el];
-                li[2 * l2] = (int)(w & 0xffffu);
-                li[2 * l2 + 1] = (int)(w >> 16);
+                h[2 * l2] = Table::of_lc(w & 0xffffu);
+                h[2 * l2 + 1] = Table::of_lc(w >> 16);
             }
 #pragma unroll
             for (int l = 0; l < 10; ++l)
 #pragma unroll
-                for (int c = 0; c < DPN; ++c) xe[l * DPN + c] = xs[li[l] * DPN + c];
-            K::apply(qds + el, kPatchElems, cl, cm, xe, ye);
+                for (int c = 0; c < DPN; ++c) xe[l * DPN + c] = tab.x(h[l], c);
+            K::apply(qds + el, kPatchElems, cl, cm, S, xe, ye);
             if (MODE == MODE_PCG) {
                 T d = T(0);
 #pragma unroll
                 for (int q = 0; q < 10 * DPN; ++q) d += xe[q] * ye[q];
-                dot += (double)d;
+                dot += (double)(d * invS);
             }
 #pragma unroll
             for (int l = 0; l < 10; ++l)
 #pragma unroll
-                for (int c = 0; c < DPN; ++c) SC::add(ys, M, li[l] * DPN + c, ye[l * DPN + c] * S);
+                for (int c = 0; c < DPN; ++c) tab.add(h[l], c, ye[l * DPN + c]);
         }
         __syncthreads();
+        if (NBUF == 2 && has_next) ok = arrive(b ^ 1);
         // 3. flush (node ids: the own range, then the foreign list still in the aux buffer)
-        for (int u = threadIdx.x; u < nloc; u += blockDim.x) {
-            const uint8_t fl = sfl[u];
-            if (HALO) {  // own nodes stored, foreign ones to their halo slots (DPN values each)
-                if (DPN == 1) {  // kept apart: the general form costs the FP32 thermal kernel 9 registers
-                    const T v = SC::take(ys, M, patch_slot(u)) * invS;
-                    if (fl & 1) continue;
-                    if (u < nown) a.y[o0 + u] = v;
-                    else a.halo[HG ? __ldg(pv.fslot + pm.fa + (u - nown)) : sfsl[u - nown]] = v;
-                    continue;
+        if (HALO) {
+            // own nodes stored, foreign ones to their halo slots (DPN values each). Dirichlet
+            // rows get a value too: no reader uses it.
+            for (int grp = threadIdx.x; grp < (o1 - n0 + V - 1) / V; grp += kPatchBS) {
+                const int j0 = n0 + V * grp;
+                const int h0 = Table::of_node(V * grp);
+                if (j0 >= o0 && j0 + V <= o1) {
+                    VT yv[DPN];
+#pragma unroll
+                    for (int e = 0; e < V; ++e)
+#pragma unroll
+                        for (int c = 0; c < DPN; ++c)
+                            reinterpret_cast<T*>(yv)[e * DPN + c] = tab.take(h0 + e * Table::kStep, c) * invS;
+#pragma unroll
+                    for (int q = 0; q < DPN; ++q) reinterpret_cast<VT*>(a.y)[(int64_t)(j0 / V) * DPN + q] = yv[q];
+                } else {
+#pragma unroll
+                    for (int e = 0; e < V; ++e)
+                        if (j0 + e >= o0 && j0 + e < o1)
+#pragma unroll
+                            for (int c = 0; c < DPN; ++c)
+                                a.y[(int64_t)(j0 + e) * DPN + c] = tab.take(h0 + e * Table::kStep, c) * invS;
                 }
-                const int64_t base = u < nown ? (int64_t)(o0 + u) * DPN
-                                              : (int64_t)(HG ? __ldg(pv.fslot + pm.fa + (u - nown)) : sfsl[u - nown]) * DPN;
-                T* dst = u < nown ? a.y : a.halo;
+            }
+            for (int i = threadIdx.x; i < pm.nfor; i += kPatchBS) {
+                const int h = Table::of_node(uf + i);
+                const int64_t at = (int64_t)(HM == 2 ? __ldg(pv.fslot + pm.fa + i) : sfsl[i]) * DPN;
+#pragma unroll
+                for (int c = 0; c < DPN; ++c) a.halo[at + c] = tab.take(h, c) * invS;
+            }
+        } else {
+            for (int u = o0 - n0 + (int)threadIdx.x; u < uf + pm.nfor; u += kPatchBS) {
+                const uint8_t fl = sfl[u];
+                const int node = u < uf ? n0 + u : sfor[u - uf];
+                const bool plain = u < uf && !(fl & kFlagShared);
+                const int h = Table::of_node(u);
 #pragma unroll
                 for (int c = 0; c < DPN; ++c) {
-                    const T v = SC::take(ys, M, patch_slot(u) * DPN + c) * invS;
-                    if (!((fl >> c) & 1)) dst[base + c] = v;
+                    const T v = tab.take(h, c) * invS;
+                    if ((fl >> c) & 1) continue;
+                    T* dst = a.y + (int64_t)node * DPN + c;
+                    if (plain) *dst = v;
+                    else atomicAdd(dst, v);
                 }
-                continue;
-            }
-            const int node = u < nown ? o0 + u : sfor[u - nown];
-            const bool plain = u < nown && !(fl & kFlagShared);
-#pragma unroll
-            for (int c = 0; c < DPN; ++c) {
-                const T v = SC::take(ys, M, patch_slot(u) * DPN + c) * invS;
-                if ((fl >> c) & 1) continue;
-                T* dst = a.y + (int64_t)node * DPN + c;
-                if (plain) *dst = v;
-                else atomicAdd(dst, v);
             }
         }
-        // The late shape needs no barrier here: the next gather writes xs and the other
-        // flag table, which no flush reads, and the accumulators are zero again.
-        if (!LATE) {
+        // Two buffers need no barrier here: the next gather writes the node values (and
+        // the other flag table), which no flush reads, and the accumulators are zero again.
+        if (NBUF == 1) {
             __syncthreads();
-            if (NBUF == 1 && threadIdx.x == 0 && has_next) {
+            if (threadIdx.x == 0 && has_next) {
                 issue_next(patch, k, 0);
                 pend |= 1u;
             }
@@ -725,22 +959,6 @@ __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
     if (MODE == MODE_PCG) {
         double v[2] = {dot, pdd};
         store_partial<2>(a.part, v);
-        if (last_block(&a.st->ticket[TICKET_PATCH])) {
-            double t[2];
-            grid_total<2>(a.part, gridDim.x, t);
-            if (threadIdx.x == 0) {
-                PcgState* st = a.st;
-                st->ticket[TICKET_PATCH] = 0;
-                const double pAp = t[0] + st->cd * t[1];
-                st->pAp = pAp;
-                if (fabs(pAp) < 1e-30) {  // iterative.rs:85
-                    st->flags |= ST_DONE | ST_BREAKDOWN;
-                    st->alpha = 0.0;  // no step: the z-form's pending x update adds nothing
-                } else {
-                    st->alpha = st->rz / pAp;
-                }
-            }
-        }
     }
 }
 
@@ -756,13 +974,15 @@ struct NodeArgs {
     const T* dinv;
     T* pbuf0;
     T* pbuf1;
-    PcgState* st;
+    PcgState* st;   // state after the node update; the start and refresh kernels work on it
+    const PcgState* st_in;  // node update: the state the patch kernel left
+    const double* part_in;  // node update: the patch kernel's partials
+    int n_in;
     double* part;
     // mixed refresh
     double* x64;
     double* w64;
     const double* b;
-    int vec;  // x, r, q, dinv, pbuf0 and pbuf1 are 16-byte aligned: k_pcg_update uses 16-byte loads
     // halo mode: foreign contributions by slot (dpn values each); node i's slots
     // follow those of nodes < i, hbase[c] = slots of nodes < 32 c, flag bits 3-6 =
     // the node's slot count
@@ -771,70 +991,6 @@ struct NodeArgs {
     const double* halo64;  // mixed refresh: FP64 slots of the FP64 apply (halo mode)
 };
 
-// 16-byte vector of T
-template <class T>
-struct Vec16;
-template <>
-struct Vec16<float> {
-    using type = float4;
-    static constexpr int N = 4;
-};
-template <>
-struct Vec16<double> {
-    using type = double2;
-    static constexpr int N = 2;
-};
-
-// x += alpha p, r -= alpha q, z = D^-1 r; r.r and r.z; stopping / refresh decision.
-// With aligned vectors (a.vec) every thread streams 16-byte loads of p, q, x, r
-// and D^-1, kUnroll vectors in flight, and a scalar loop covers the tail.
-// r.r and r.z partials of the node update; the last block sums them, tests
-// convergence (FP64) or the refresh criteria (mixed) and sets beta.
-template <class T, bool MIXED>
-__device__ __forceinline__ void pcg_update_finish(const NodeArgs<T>& a, T acc_rr, T acc_rz) {
-    PcgState* st = a.st;
-    double v[2] = {(double)acc_rr, (double)acc_rz};
-    store_partial<2>(a.part, v);
-    if (last_block(&st->ticket[TICKET_UPDATE])) {
-        double t[2];
-        grid_total<2>(a.part, gridDim.x, t);
-        if (threadIdx.x == 0) {
-            st->ticket[TICKET_UPDATE] = 0;
-            const double rn = sqrt(t[0]);
-            if (!MIXED) {
-                st->res = rn;
-                if (rn < st->tol * st->bnorm || rn < st->abs_tol) {  // iterative.rs:95
-                    st->flags |= ST_DONE | ST_CONVERGED;
-                    return;
-                }
-            }
-            st->beta = t[1] / st->rz;
-            st->rz_old = st->rz;
-            st->rz = t[1];
-            st->it += 1;
-            if (MIXED) {
-                st->rmax = fmax(st->rmax, rn);
-                const double est = rn * st->s_scale;
-                if (est < st->tol * st->bnorm || est < st->abs_tol || rn < st->delta * st->rmax ||
-                    st->it >= st->max_it)
-                    st->flags |= ST_REFRESH;
-            } else if (st->it >= st->max_it) {
-                st->flags |= ST_DONE;
-            }
-        }
-    }
-}
-
-// k_pcg_update_halo: one 16-byte vector per array in flight per thread, four
-// resident blocks (64 registers; the z-form: six, below). The halo loads wait on the slot scan, so warps
-// hide that latency better than deeper unrolling: at 128^3 (FP32) 0.095 ms
-// against 0.107 ms (two vectors) and 0.20 ms (four, one block per SM).
-// The z-form update of the mixed thermal solver streams four vectors instead of
-// seven and fits six blocks per SM (42 registers): 0.073 ms at 128^3 against
-// 0.085 ms at four blocks and 0.081 ms at eight.
-constexpr int kHaloUnroll = 1;
-constexpr int kHaloMinBlocks = 4;
-constexpr int kHaloMinBlocksZ = 6;
 constexpr int kHaloShift = 3;  // flag bits 3-6: halo slots of the node (halo mode)
 
 // ro / dj for the norms of the z-form (FP32: the fast reciprocal-multiply, within
@@ -842,24 +998,69 @@ constexpr int kHaloShift = 3;  // flag bits 3-6: halo slots of the node (halo mo
 __device__ __forceinline__ float fast_div(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double fast_div(double a, double b) { return a / b; }
 
-// Sum of node j's halo slots, starting at slot s (fixed order: slot order).
+// The axpys of one row: x += alpha p, r -= alpha q (Dirichlet rows q = cd p), z = D^-1 r,
+// and its terms of r.r and r.z. ZF (the mixed solver's z-form, see k_patch): r holds
+// z = D^-1 r, x is not touched (the next patch kernel updates it).
+template <class T, bool ZF>
+struct PcgRow {
+    T alpha, cd;
+    T rr = T(0), rz = T(0);
+    __device__ __forceinline__ void operator()(bool dir, T p, T q, T dinv, T& x, T& r) {
+        const T qq = dir ? cd * p : q;
+        if (ZF) {
+            r = r - alpha * (dinv * qq);
+            const T v = fast_div(r, dinv);
+            rr += v * v;
+            rz += v * r;
+            return;
+        }
+        x = x + alpha * p;
+        r = r - alpha * qq;
+        rr += r * r;
+        rz += r * (r * dinv);
+    }
+};
+
+// Folds the patch kernel's partials in (see pcg_fold).
 template <class T>
-__device__ __forceinline__ T halo_sum(const T* __restrict__ halo, int64_t s, int cnt) {
-    T h = T(0);
-    for (int i = 0; i < cnt; ++i) h += halo[s + i];
-    return h;
+__device__ __forceinline__ PcgHead pcg_fold_patch(const NodeArgs<T>& a) {
+    return pcg_fold(a.st_in, a.st, a.part_in, a.n_in,
+                    [](PcgScalars& s, double t0, double t1) { pcg_step_length(s, t0, t1); });
 }
 
-// Node update of a one-DOF operator in halo mode: as the loops of k_pcg_update,
-// with q_j = (own-patch sum, stored by the patch kernel) + (node j's halo slots).
-// Lane l of a warp takes vector iv (V nodes); the warp's 32 vectors are 32 V
-// consecutive nodes starting at a multiple of 32, so its first slot is
-// hbase[first / 32] and each lane's first slot follows from a warp scan of the
-// lanes' slot counts. Loop conditions are warp-uniform (lanes past the end load
-// nothing and count 0 slots).
-template <class T, int kU, bool ZF>
-__device__ __forceinline__ void pcg_update_halo(const NodeArgs<T>& a, T alpha, T cd, const T* __restrict__ p,
-                                                T& acc_rr, T& acc_rz) {
+// Exclusive prefix over the warp of the lanes' slot counts: added to the slots before
+// the warp's first node (hbase) it gives a lane's first halo slot. Every lane of the
+// warp calls it (lanes past the end pass cnt = 0).
+__device__ __forceinline__ int halo_prefix(int cnt, int lane) {
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    return incl - cnt;
+}
+
+// First halo slot of node j alone, from the start of its 32-node chunk.
+__device__ __forceinline__ int64_t halo_first(const uint8_t* __restrict__ flags, const int32_t* __restrict__ hbase,
+                                              int64_t j) {
+    int64_t s = hbase[j / 32];
+    for (int64_t i = j & ~(int64_t)31; i < j; ++i) s += (flags[i] >> kHaloShift) & 15;
+    return s;
+}
+
+// Node update of a one-DOF operator in halo mode: q_j = (own-patch sum, stored by the
+// patch kernel) + (node j's halo slots, in slot order). Lane l of a warp takes vector
+// iv (V nodes); the warp's 32 vectors are 32 V consecutive nodes starting at a multiple
+// of 32, so its first slot is hbase[first / 32] and each lane's follows from a warp
+// scan of the lanes' slot counts. Loop conditions are warp-uniform.
+// The first vector's loads, slot scan and halo sums are issued before the partials of
+// the patch kernel are folded in: they need none of the iteration's scalars. One
+// vector per array in flight per thread: the halo loads wait on the slot scan, so
+// warps hide that latency better than deeper unrolling (two vectors 0.107, four 0.20
+// against 0.095 ms at 128^3, FP32).
+template <class T, bool ZF>
+__device__ __forceinline__ bool pcg_update_halo(const NodeArgs<T>& a, PcgRow<T, ZF>& row) {
     using VT = typename Vec16<T>::type;
     constexpr int V = Vec16<T>::N;
     const uint8_t* __restrict__ flags = a.flags;
@@ -868,133 +1069,214 @@ __device__ __forceinline__ void pcg_update_halo(const NodeArgs<T>& a, T alpha, T
     T* __restrict__ x = a.x;
     T* __restrict__ r = a.r;
     const T* __restrict__ q = a.q;
+    const T* __restrict__ p = (a.st_in->it & 1) ? a.pbuf0 : a.pbuf1;
     const int lane = threadIdx.x & 31;
     const int64_t n = a.n, nth = (int64_t)gridDim.x * blockDim.x;
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    // ZF (mixed solver's z-form, see k_patch): r holds z = D^-1 r, x is not touched
-    // (the next patch kernel updates it) and p is read only where a Dirichlet row needs it
-    auto entry = [&](T pj, T qj, T xj, T rj, T dj, uint8_t f, T& xo, T& ro) {
-        const T qq = (f & 1) ? cd * pj : qj;
-        if (ZF) {
-            ro = rj - alpha * (dj * qq);
-            const T rr = fast_div(ro, dj);
-            acc_rr += rr * rr;
-            acc_rz += rr * ro;
-            xo = xj;
-            return;
-        }
-        xo = xj + alpha * pj;
-        ro = rj - alpha * qq;
-        acc_rr += ro * ro;
-        acc_rz += ro * (ro * dj);
-    };
-    // first slot of this lane's V nodes; every lane of the warp calls it
-    auto lane_slot = [&](int64_t iv, int tot) {
-        int incl = tot;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const int64_t first = __shfl_sync(0xffffffffu, iv, 0) * V;
-        return (int64_t)a.hbase[first / 32] + (incl - tot);
-    };
-    const int64_t nv = a.vec ? n / V : 0;
-    int64_t iv = tid;
-    for (; iv - lane + 31 + (kU - 1) * nth < nv; iv += kU * nth) {  // all lanes, all u in range
-        VT pv[kU] = {}, qv[kU], xv[kU], rv[kU], dv[kU];
-        uint8_t fl[kU][V];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int64_t k = iv + u * nth;
-            qv[u] = reinterpret_cast<const VT*>(q)[k];
-            if (!ZF) xv[u] = reinterpret_cast<const VT*>(x)[k];
-            rv[u] = reinterpret_cast<const VT*>(r)[k];
-            dv[u] = reinterpret_cast<const VT*>(dinv)[k];
-            uint8_t any_dir = 0;
-#pragma unroll
-            for (int e = 0; e < V; ++e) {
-                fl[u][e] = flags[k * V + e];
-                any_dir |= fl[u][e];
-            }
-            if (!ZF || (any_dir & 1)) pv[u] = reinterpret_cast<const VT*>(p)[k];
-        }
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int64_t k = iv + u * nth;
-            int cnt[V], tot = 0;
-#pragma unroll
-            for (int e = 0; e < V; ++e) {
-                cnt[e] = (fl[u][e] >> kHaloShift) & 15;
-                tot += cnt[e];
-            }
-            int64_t sl = lane_slot(k, tot);
-            const T* pe = reinterpret_cast<const T*>(&pv[u]);
-            const T* qe = reinterpret_cast<const T*>(&qv[u]);
-            const T* xe = reinterpret_cast<const T*>(&xv[u]);
-            const T* re = reinterpret_cast<const T*>(&rv[u]);
-            const T* de = reinterpret_cast<const T*>(&dv[u]);
-            VT xo, ro;
-            T* xoe = reinterpret_cast<T*>(&xo);
-            T* roe = reinterpret_cast<T*>(&ro);
-#pragma unroll
-            for (int e = 0; e < V; ++e) {
-                const T qj = qe[e] + halo_sum(halo, sl, cnt[e]);
-                sl += cnt[e];
-                entry(pe[e], qj, xe[e], re[e], de[e], fl[u][e], xoe[e], roe[e]);
-            }
-            if (!ZF) reinterpret_cast<VT*>(x)[k] = xo;
-            reinterpret_cast<VT*>(r)[k] = ro;
-        }
-    }
-    for (; iv - lane < nv; iv += nth) {  // warp-uniform: some lanes may be past nv
+    const int64_t nv = n / V;
+    VT pv, qv, xv, rv, dv;
+    unsigned dir;  // bit e: entry e is a Dirichlet row
+    auto load = [&](int64_t iv) {
         const bool in = iv < nv;
-        uint8_t fl[V];
         int cnt[V], tot = 0;
+        dir = 0;
+        if (in) {
+            qv = reinterpret_cast<const VT*>(q)[iv];
+            if (!ZF) xv = reinterpret_cast<const VT*>(x)[iv];
+            rv = reinterpret_cast<const VT*>(r)[iv];
+            dv = reinterpret_cast<const VT*>(dinv)[iv];
+            if (!ZF) pv = reinterpret_cast<const VT*>(p)[iv];
+        }
 #pragma unroll
         for (int e = 0; e < V; ++e) {
-            fl[e] = in ? flags[iv * V + e] : (uint8_t)0;
-            cnt[e] = (fl[e] >> kHaloShift) & 15;
+            const uint8_t f = in ? flags[iv * V + e] : (uint8_t)0;
+            dir |= (unsigned)(f & 1) << e;
+            cnt[e] = (f >> kHaloShift) & 15;
             tot += cnt[e];
         }
-        int64_t sl = lane_slot(iv, tot);
-        if (in) {
-            const VT pv = reinterpret_cast<const VT*>(p)[iv], qv = reinterpret_cast<const VT*>(q)[iv];
-            const VT xv = ZF ? VT{} : reinterpret_cast<const VT*>(x)[iv], rv = reinterpret_cast<const VT*>(r)[iv];
-            const VT dv = reinterpret_cast<const VT*>(dinv)[iv];
-            VT xo, ro;
+        const int64_t first = (iv - lane) * V;
+        int64_t sl = (int64_t)a.hbase[first / 32] + halo_prefix(tot, lane);
+        T* qe = reinterpret_cast<T*>(&qv);
 #pragma unroll
-            for (int e = 0; e < V; ++e) {
-                const T qj = reinterpret_cast<const T*>(&qv)[e] + halo_sum(halo, sl, cnt[e]);
-                sl += cnt[e];
-                entry(reinterpret_cast<const T*>(&pv)[e], qj, reinterpret_cast<const T*>(&xv)[e],
-                      reinterpret_cast<const T*>(&rv)[e], reinterpret_cast<const T*>(&dv)[e], fl[e],
-                      reinterpret_cast<T*>(&xo)[e], reinterpret_cast<T*>(&ro)[e]);
-            }
-            if (!ZF) reinterpret_cast<VT*>(x)[iv] = xo;
-            reinterpret_cast<VT*>(r)[iv] = ro;
+        for (int e = 0; e < V; ++e) {
+            T h = T(0);
+            for (int i = 0; i < cnt[e]; ++i) h += halo[sl + i];
+            sl += cnt[e];
+            qe[e] += h;
         }
+    };
+    int64_t iv = tid;
+    if (iv - lane < nv) load(iv);
+    const PcgHead h = pcg_fold_patch(a);
+    if (h.flags & (ST_DONE | ST_REFRESH)) return false;
+    row.alpha = (T)h.alpha;
+    row.cd = (T)h.cd;
+    while (iv - lane < nv) {
+        if (iv < nv) {
+            if (ZF && dir) pv = reinterpret_cast<const VT*>(p)[iv];  // z-form: p only where a Dirichlet row needs it
+#pragma unroll
+            for (int e = 0; e < V; ++e)
+                row((dir >> e) & 1, reinterpret_cast<T*>(&pv)[e], reinterpret_cast<T*>(&qv)[e],
+                    reinterpret_cast<T*>(&dv)[e], reinterpret_cast<T*>(&xv)[e], reinterpret_cast<T*>(&rv)[e]);
+            if (!ZF) reinterpret_cast<VT*>(x)[iv] = xv;
+            reinterpret_cast<VT*>(r)[iv] = rv;
+        }
+        iv += nth;
+        if (iv - lane < nv) load(iv);
     }
-    // the last n mod V nodes (all nodes when the vectors are not 16-byte aligned):
-    // the slot base from the 32-node chunk start
-    for (int64_t j = nv * V + tid; j < n; j += nth) {
+    for (int64_t j = nv * V + tid; j < n; j += nth) {  // the last n mod V nodes
         const uint8_t f = flags[j];
-        int64_t sl = a.hbase[j / 32];
-        for (int64_t i = j & ~(int64_t)31; i < j; ++i) sl += (flags[i] >> kHaloShift) & 15;
-        T xo, ro;
-        entry(p[j], q[j] + halo_sum(halo, sl, (f >> kHaloShift) & 15), ZF ? T(0) : x[j], r[j], dinv[j], f, xo, ro);
+        const int64_t sl = halo_first(flags, a.hbase, j);
+        T hs = T(0), xo = ZF ? T(0) : x[j], ro = r[j];
+        for (int i = 0; i < ((f >> kHaloShift) & 15); ++i) hs += halo[sl + i];
+        row(f & 1, p[j], q[j] + hs, dinv[j], xo, ro);
         if (!ZF) x[j] = xo;
         r[j] = ro;
     }
+    return true;
 }
 
+// Node update of a three-DOF operator in halo mode, as pcg_update_halo. FP32: two
+// consecutive nodes per lane, so that each vector's six values are three 8-byte loads
+// (a lane's pair starts at DOF 6 m) and a warp covers 64 nodes starting at a multiple
+// of 64; FP64: one node per lane.
+template <class T, bool ZF>
+__device__ __forceinline__ bool pcg_update_halo3(const NodeArgs<T>& a, PcgRow<T, ZF>& row) {
+    constexpr int P = std::is_same_v<T, float> ? 2 : 1;  // nodes per lane
+    const uint8_t* __restrict__ flags = a.flags;
+    const T* __restrict__ dinv = a.dinv;
+    const T* __restrict__ halo = a.halo;
+    T* __restrict__ x = a.x;
+    T* __restrict__ r = a.r;
+    const T* __restrict__ q = a.q;
+    const T* __restrict__ p = (a.st_in->it & 1) ? a.pbuf0 : a.pbuf1;
+    const int lane = threadIdx.x & 31;
+    const int64_t nn = a.n / 3, nth = (int64_t)gridDim.x * blockDim.x;
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t nm = nn / P;
+    T pv[3 * P], qv[3 * P], xv[3 * P], rv[3 * P], dv[3 * P];
+    unsigned f[P];
+    auto get = [&](const T* __restrict__ src, int64_t m, T (&v)[3 * P]) {
+        if constexpr (P == 2) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float2 t = reinterpret_cast<const float2*>(src)[3 * m + k];
+                v[2 * k] = t.x, v[2 * k + 1] = t.y;
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[c] = src[3 * m + c];
+        }
+    };
+    auto put = [&](T* __restrict__ dst, int64_t m, const T (&v)[3 * P]) {
+        if constexpr (P == 2) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) reinterpret_cast<float2*>(dst)[3 * m + k] = make_float2(v[2 * k], v[2 * k + 1]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) dst[3 * m + c] = v[c];
+        }
+    };
+    auto load = [&](int64_t m) {
+        const bool in = m < nm;
+        int tot = 0;
+#pragma unroll
+        for (int e = 0; e < P; ++e) {
+            f[e] = in ? flags[P * m + e] : 0u;
+            tot += (f[e] >> kHaloShift) & 15;
+        }
+        if (in) {
+            get(q, m, qv);
+            if (!ZF) get(x, m, xv);
+            get(r, m, rv);
+            get(dinv, m, dv);
+            if (!ZF) get(p, m, pv);
+        }
+        const int64_t first = (m - lane) * P;
+        int64_t sl = (int64_t)a.hbase[first / 32] + halo_prefix(tot, lane);
+#pragma unroll
+        for (int e = 0; e < P; ++e) {
+            const int cnt = (f[e] >> kHaloShift) & 15;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                T h = T(0);
+                for (int i = 0; i < cnt; ++i) h += halo[3 * (sl + i) + c];
+                qv[3 * e + c] += h;
+            }
+            sl += cnt;
+        }
+    };
+    int64_t m = tid;
+    if (m - lane < nm) load(m);
+    const PcgHead h = pcg_fold_patch(a);
+    if (h.flags & (ST_DONE | ST_REFRESH)) return false;
+    row.alpha = (T)h.alpha;
+    row.cd = (T)h.cd;
+    while (m - lane < nm) {
+        if (m < nm) {
+            // z-form: p only where a Dirichlet row needs it
+            if (ZF && ((f[0] | f[P - 1]) & 7u)) get(p, m, pv);
+#pragma unroll
+            for (int e = 0; e < P; ++e)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const int v = 3 * e + c;
+                    row((f[e] >> c) & 1, pv[v], qv[v], dv[v], xv[v], rv[v]);
+                }
+            if (!ZF) put(x, m, xv);
+            put(r, m, rv);
+        }
+        m += nth;
+        if (m - lane < nm) load(m);
+    }
+    for (int64_t nd = P * nm + tid; nd < nn; nd += nth) {  // an odd last node
+        const unsigned fl = flags[nd];
+        const int cnt = (fl >> kHaloShift) & 15;
+        const int64_t sl = halo_first(flags, a.hbase, nd);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int64_t j = 3 * nd + c;
+            T hs = T(0), xo = ZF ? T(0) : x[j], ro = r[j];
+            for (int i = 0; i < cnt; ++i) hs += halo[3 * (sl + i) + c];
+            row((fl >> c) & 1, p[j], q[j] + hs, dinv[j], xo, ro);
+            if (!ZF) x[j] = xo;
+            r[j] = ro;
+        }
+    }
+    return true;
+}
+
+// Resident blocks per SM of the halo-mode node update: four (64 registers); the z-form
+// of the mixed thermal solver streams four vectors instead of seven and fits six (40
+// registers): 0.069 ms at 128^3 against 0.072 ms at five and 0.086 ms at four blocks.
+constexpr int kHaloMinBlocks = 4;
+constexpr int kHaloMinBlocksZ = 6;
+
+// Node update of a PCG in halo mode (see pcg_update_halo / pcg_update_halo3).
+template <class T, int DPN, bool MIXED>
+__global__ void __launch_bounds__(kNodeBS, (MIXED && DPN == 1 && std::is_same<T, float>::value) ? kHaloMinBlocksZ
+                                                                                             : kHaloMinBlocks)
+    k_pcg_update_halo(NodeArgs<T> a) {
+    PcgRow<T, MIXED && std::is_same<T, float>::value> row;
+    if (DPN == 1) {
+        if (!pcg_update_halo(a, row)) return;
+    } else {
+        if (!pcg_update_halo3(a, row)) return;
+    }
+    double v[2] = {(double)row.rr, (double)row.rz};
+    store_partial<2>(a.part, v);
+}
+
+// Node update in atomics mode (a mesh with a node of more than 15 foreign entries):
+// every thread streams 16-byte vectors of p, q, x, r and D^-1, kUnroll in flight, and a
+// scalar loop covers the tail. q is zeroed where another patch accumulates into it in
+// the next iteration.
 template <class T, int DPN, bool MIXED>
 __global__ void __launch_bounds__(kNodeBS) k_pcg_update(NodeArgs<T> a) {
-    PcgState* st = a.st;
-    if (st->flags & (ST_DONE | ST_REFRESH)) return;
-    const T alpha = (T)st->alpha;
-    const T cd = (T)st->cd;
-    const T* __restrict__ p = (st->it & 1) ? a.pbuf0 : a.pbuf1;
+    constexpr bool ZF = MIXED && std::is_same<T, float>::value;
+    const PcgHead h = pcg_fold_patch(a);
+    if (h.flags & (ST_DONE | ST_REFRESH)) return;
+    const T* __restrict__ p = h.odd ? a.pbuf0 : a.pbuf1;
     const uint8_t* __restrict__ flags = a.flags;
     const T* __restrict__ dinv = a.dinv;
     T* __restrict__ x = a.x;
@@ -1004,30 +1286,16 @@ __global__ void __launch_bounds__(kNodeBS) k_pcg_update(NodeArgs<T> a) {
     constexpr int V = Vec16<T>::N;
     const int64_t n = a.n, nth = (int64_t)gridDim.x * blockDim.x;
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    T acc_rr = T(0), acc_rz = T(0);
-    // z-form (the mixed solver, see k_patch): r holds z = D^-1 r and x is updated by the
-    // next patch kernel
-    constexpr bool ZF = MIXED && std::is_same<T, float>::value;
-    // one entry: new x and r (z-form: new z), q zeroed where another patch accumulates into it next time
-    auto entry = [&](int64_t j, T pj, T qj, T xj, T rj, T dj, T& xo, T& ro) {
+    PcgRow<T, ZF> row;
+    row.alpha = (T)h.alpha;
+    row.cd = (T)h.cd;
+    auto entry = [&](int64_t j, T pj, T qj, T dj, T& xj, T& rj) {
         const uint8_t f = flags[j / DPN];
         const bool dir = (f >> (j % DPN)) & 1;
-        const T qq = dir ? cd * pj : qj;
         if (!dir && (f & kFlagShared)) q[j] = T(0);
-        if (ZF) {
-            ro = rj - alpha * (dj * qq);
-            const T rr = fast_div(ro, dj);
-            acc_rr += rr * rr;
-            acc_rz += rr * ro;
-            xo = xj;
-            return;
-        }
-        xo = xj + alpha * pj;
-        ro = rj - alpha * qq;
-        acc_rr += ro * ro;
-        acc_rz += ro * (ro * dj);
+        row(dir, pj, qj, dj, xj, rj);
     };
-    const int64_t nv = a.vec ? n / V : 0;
+    const int64_t nv = n / V;
     int64_t iv = tid;
     for (; iv + (kUnroll - 1) * nth < nv; iv += kUnroll * nth) {
         VT pv[kUnroll], qv[kUnroll], xv[kUnroll], rv[kUnroll], dv[kUnroll];
@@ -1043,221 +1311,32 @@ __global__ void __launch_bounds__(kNodeBS) k_pcg_update(NodeArgs<T> a) {
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
             const int64_t k = iv + u * nth;
-            const T* pe = reinterpret_cast<const T*>(&pv[u]);
-            const T* qe = reinterpret_cast<const T*>(&qv[u]);
-            const T* xe = reinterpret_cast<const T*>(&xv[u]);
-            const T* re = reinterpret_cast<const T*>(&rv[u]);
-            const T* de = reinterpret_cast<const T*>(&dv[u]);
-            VT xo, ro;
-            T* xoe = reinterpret_cast<T*>(&xo);
-            T* roe = reinterpret_cast<T*>(&ro);
 #pragma unroll
-            for (int e = 0; e < V; ++e) entry(k * V + e, pe[e], qe[e], xe[e], re[e], de[e], xoe[e], roe[e]);
-            if (!ZF) reinterpret_cast<VT*>(x)[k] = xo;
-            reinterpret_cast<VT*>(r)[k] = ro;
+            for (int e = 0; e < V; ++e)
+                entry(k * V + e, reinterpret_cast<const T*>(&pv[u])[e], reinterpret_cast<const T*>(&qv[u])[e],
+                      reinterpret_cast<const T*>(&dv[u])[e], reinterpret_cast<T*>(&xv[u])[e],
+                      reinterpret_cast<T*>(&rv[u])[e]);
+            if (!ZF) reinterpret_cast<VT*>(x)[k] = xv[u];
+            reinterpret_cast<VT*>(r)[k] = rv[u];
         }
     }
-    for (; iv < nv; iv += nth) {
-        const VT pv = reinterpret_cast<const VT*>(p)[iv], qv = reinterpret_cast<const VT*>(q)[iv];
-        const VT xv = ZF ? VT{} : reinterpret_cast<const VT*>(x)[iv], rv = reinterpret_cast<const VT*>(r)[iv];
-        const VT dv = reinterpret_cast<const VT*>(dinv)[iv];
-        VT xo, ro;
-#pragma unroll
-        for (int e = 0; e < V; ++e)
-            entry(iv * V + e, reinterpret_cast<const T*>(&pv)[e], reinterpret_cast<const T*>(&qv)[e],
-                  reinterpret_cast<const T*>(&xv)[e], reinterpret_cast<const T*>(&rv)[e],
-                  reinterpret_cast<const T*>(&dv)[e], reinterpret_cast<T*>(&xo)[e], reinterpret_cast<T*>(&ro)[e]);
-        if (!ZF) reinterpret_cast<VT*>(x)[iv] = xo;
-        reinterpret_cast<VT*>(r)[iv] = ro;
-    }
+    // the remaining vectors and the last n mod V entries
+    for (int64_t k = iv; k < nv; k += nth)
+        for (int e = 0; e < V; ++e) {
+            const int64_t j = k * V + e;
+            T xj = ZF ? T(0) : x[j], rj = r[j];
+            entry(j, p[j], q[j], dinv[j], xj, rj);
+            if (!ZF) x[j] = xj;
+            r[j] = rj;
+        }
     for (int64_t j = nv * V + tid; j < n; j += nth) {
-        T xo, ro;
-        entry(j, p[j], q[j], ZF ? T(0) : x[j], r[j], dinv[j], xo, ro);
-        if (!ZF) x[j] = xo;
-        r[j] = ro;
+        T xj = ZF ? T(0) : x[j], rj = r[j];
+        entry(j, p[j], q[j], dinv[j], xj, rj);
+        if (!ZF) x[j] = xj;
+        r[j] = rj;
     }
-    pcg_update_finish<T, MIXED>(a, acc_rr, acc_rz);
-}
-
-// Node update of a three-DOF operator in halo mode: one node per lane, its three
-// interleaved DOFs of every vector by scalar loads (issued before the slot scan),
-// then its slots' three components. A warp's 32 lanes are 32 consecutive nodes
-// starting at a multiple of 32, as in pcg_update_halo.
-template <class T, bool ZF>
-__device__ __forceinline__ void pcg_update_halo3(const NodeArgs<T>& a, T alpha, T cd, const T* __restrict__ p,
-                                                 T& acc_rr, T& acc_rz) {
-    const uint8_t* __restrict__ flags = a.flags;
-    const T* __restrict__ dinv = a.dinv;
-    const T* __restrict__ halo = a.halo;
-    T* __restrict__ x = a.x;
-    T* __restrict__ r = a.r;
-    const T* __restrict__ q = a.q;
-    const int lane = threadIdx.x & 31;
-    const int64_t nn = a.n / 3, nth = (int64_t)gridDim.x * blockDim.x;
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if constexpr (std::is_same_v<T, float>) {
-        if (a.vec) {
-            // FP32: two consecutive nodes per lane, so that each vector's six values are
-            // three 8-byte loads (a lane's pair starts at DOF 6 m); a warp covers 64
-            // nodes starting at a multiple of 64
-            const int64_t np2 = nn / 2;
-            for (int64_t m = tid; m - lane < np2; m += nth) {
-                const bool in = m < np2;
-                float pv[6], qv[6], xv[6], rv[6], dv[6];
-                uint8_t f[2] = {0, 0};
-                if (in) {
-                    f[0] = flags[2 * m];
-                    f[1] = flags[2 * m + 1];
-                    // z-form: p only where a Dirichlet row needs it, x not touched
-                    const bool need_p = !ZF || ((f[0] | f[1]) & 7);
-    #pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        const float2 tp = need_p ? reinterpret_cast<const float2*>(p)[3 * m + k] : make_float2(0.f, 0.f);
-                        const float2 tq = reinterpret_cast<const float2*>(q)[3 * m + k];
-                        const float2 tx = ZF ? make_float2(0.f, 0.f) : reinterpret_cast<const float2*>(x)[3 * m + k];
-                        const float2 tr = reinterpret_cast<const float2*>(r)[3 * m + k];
-                        const float2 td = reinterpret_cast<const float2*>(dinv)[3 * m + k];
-                        pv[2 * k] = tp.x, pv[2 * k + 1] = tp.y;
-                        qv[2 * k] = tq.x, qv[2 * k + 1] = tq.y;
-                        xv[2 * k] = tx.x, xv[2 * k + 1] = tx.y;
-                        rv[2 * k] = tr.x, rv[2 * k + 1] = tr.y;
-                        dv[2 * k] = td.x, dv[2 * k + 1] = td.y;
-                    }
-                }
-                const int c0 = (f[0] >> kHaloShift) & 15, c1 = (f[1] >> kHaloShift) & 15;
-                const int tot = c0 + c1;
-                int incl = tot;
-    #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += t;
-                }
-                const int64_t first = __shfl_sync(0xffffffffu, m, 0) * 2;
-                const int64_t s0 = (int64_t)a.hbase[first / 32] + (incl - tot);
-                if (!in) continue;
-    #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int cnt = e ? c1 : c0;
-                    const int64_t se = s0 + (e ? c0 : 0);
-    #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const int v = 3 * e + c;
-                        float h = 0.0f;
-                        for (int i = 0; i < cnt; ++i) h += halo[3 * (se + i) + c];
-                        const float qq = ((f[e] >> c) & 1) ? (float)cd * pv[v] : qv[v] + h;
-                        if (ZF) {  // rv holds z = D^-1 r
-                            rv[v] = rv[v] - (float)alpha * (dv[v] * qq);
-                            const float rr = fast_div(rv[v], dv[v]);
-                            acc_rr += rr * rr;
-                            acc_rz += rr * rv[v];
-                            continue;
-                        }
-                        xv[v] = xv[v] + (float)alpha * pv[v];
-                        rv[v] = rv[v] - (float)alpha * qq;
-                        acc_rr += rv[v] * rv[v];
-                        acc_rz += rv[v] * (rv[v] * dv[v]);
-                    }
-                }
-    #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    if (!ZF) reinterpret_cast<float2*>(x)[3 * m + k] = make_float2(xv[2 * k], xv[2 * k + 1]);
-                    reinterpret_cast<float2*>(r)[3 * m + k] = make_float2(rv[2 * k], rv[2 * k + 1]);
-                }
-            }
-            // an odd last node: its first slot from the 32-node chunk start
-            for (int64_t nd = 2 * np2 + tid; nd < nn; nd += nth) {
-                const uint8_t f = flags[nd];
-                const int cnt = (f >> kHaloShift) & 15;
-                int64_t s0 = a.hbase[nd / 32];
-                for (int64_t i = nd & ~(int64_t)31; i < nd; ++i) s0 += (flags[i] >> kHaloShift) & 15;
-    #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const int64_t j = 3 * nd + c;
-                    T h = T(0);
-                    for (int i = 0; i < cnt; ++i) h += halo[3 * (s0 + i) + c];
-                    const T qq = ((f >> c) & 1) ? cd * p[j] : q[j] + h;
-                    if (ZF) {
-                        const T zo = r[j] - alpha * (dinv[j] * qq);
-                        const T rr = fast_div(zo, dinv[j]);
-                        r[j] = zo;
-                        acc_rr += rr * rr;
-                        acc_rz += rr * zo;
-                        continue;
-                    }
-                    const T xo = x[j] + alpha * p[j];
-                    const T ro = r[j] - alpha * qq;
-                    x[j] = xo;
-                    r[j] = ro;
-                    acc_rr += ro * ro;
-                    acc_rz += ro * (ro * dinv[j]);
-                }
-            }
-            return;
-        }
-    }
-    for (int64_t nd = tid; nd - lane < nn; nd += nth) {
-        const bool in = nd < nn;
-        T pv[3], qv[3], xv[3], rv[3], dv[3];
-        uint8_t f = 0;
-        if (in) {
-            f = flags[nd];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const int64_t j = 3 * nd + c;
-                pv[c] = p[j];
-                qv[c] = q[j];
-                xv[c] = ZF ? T(0) : x[j];
-                rv[c] = r[j];
-                dv[c] = dinv[j];
-            }
-        }
-        const int cnt = (f >> kHaloShift) & 15;
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const int64_t first = __shfl_sync(0xffffffffu, nd, 0);
-        const int64_t s0 = (int64_t)a.hbase[first / 32] + (incl - cnt);
-        if (!in) continue;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            T h = T(0);
-            for (int i = 0; i < cnt; ++i) h += halo[3 * (s0 + i) + c];
-            const T qq = ((f >> c) & 1) ? cd * pv[c] : qv[c] + h;
-            if (ZF) {
-                const T zo = rv[c] - alpha * (dv[c] * qq);
-                const T rr = fast_div(zo, dv[c]);
-                r[3 * nd + c] = zo;
-                acc_rr += rr * rr;
-                acc_rz += rr * zo;
-                continue;
-            }
-            const T xo = xv[c] + alpha * pv[c];
-            const T ro = rv[c] - alpha * qq;
-            x[3 * nd + c] = xo;
-            r[3 * nd + c] = ro;
-            acc_rr += ro * ro;
-            acc_rz += ro * (ro * dv[c]);
-        }
-    }
-}
-
-// Node update of a PCG in halo mode (see pcg_update_halo / pcg_update_halo3).
-template <class T, int DPN, bool MIXED>
-__global__ void __launch_bounds__(kNodeBS, (MIXED && DPN == 1 && std::is_same<T, float>::value) ? kHaloMinBlocksZ
-                                                                                             : kHaloMinBlocks)
-    k_pcg_update_halo(NodeArgs<T> a) {
-    PcgState* st = a.st;
-    if (st->flags & (ST_DONE | ST_REFRESH)) return;
-    const T* __restrict__ p = (st->it & 1) ? a.pbuf0 : a.pbuf1;
-    T acc_rr = T(0), acc_rz = T(0);
-    if (DPN == 1)
-        pcg_update_halo<T, kHaloUnroll, MIXED && std::is_same<T, float>::value>(a, (T)st->alpha, (T)st->cd, p,
-                                                                                 acc_rr, acc_rz);
-    else pcg_update_halo3<T, MIXED && std::is_same<T, float>::value>(a, (T)st->alpha, (T)st->cd, p, acc_rr, acc_rz);
-    pcg_update_finish<T, MIXED>(a, acc_rr, acc_rz);
+    double v[2] = {(double)row.rr, (double)row.rz};
+    store_partial<2>(a.part, v);
 }
 
 // FP64 mode start: x = 0, r = b, p_old = 0, q = 0; ||b||, r.z.
@@ -1276,17 +1355,18 @@ __global__ void __launch_bounds__(kNodeBS) k_pcg_init(NodeArgs<T> a) {
     }
     double v[2] = {bb, rz};
     store_partial<2>(a.part, v);
-    if (last_block(&a.st->ticket[TICKET_AUX])) {
+    if (last_block(&a.st->ticket)) {
         double t[2];
         grid_total<2>(a.part, gridDim.x, t);
         if (threadIdx.x == 0) {
             PcgState* st = a.st;
-            st->ticket[TICKET_AUX] = 0;
+            st->ticket = 0;
             st->bnorm = sqrt(t[0]);
             st->res = st->bnorm;
             st->rz = t[1];
             st->beta = 0.0;
             st->it = 0;
+            st->pending = 0;
             st->nupd = 0;
             st->s_scale = 1.0;
             st->rmax = 1.0;
@@ -1314,17 +1394,18 @@ __global__ void __launch_bounds__(kNodeBS) k_mixed_init1(NodeArgs<float> a) {
     }
     double v[1] = {bb};
     store_partial<1>(a.part, v);
-    if (last_block(&a.st->ticket[TICKET_AUX])) {
+    if (last_block(&a.st->ticket)) {
         double t[1];
         grid_total<1>(a.part, gridDim.x, t);
         if (threadIdx.x == 0) {
             PcgState* st = a.st;
-            st->ticket[TICKET_AUX] = 0;
+            st->ticket = 0;
             st->bnorm = sqrt(t[0]);
             st->res = st->bnorm;
             st->s_scale = st->bnorm;
             st->beta = 0.0;
             st->it = 0;
+            st->pending = 0;
             st->nupd = 0;
             st->rmax = 1.0;
             if (st->bnorm < 1e-25) {
@@ -1351,11 +1432,11 @@ __global__ void __launch_bounds__(kNodeBS) k_mixed_init2(NodeArgs<float> a) {
     }
     double v[1] = {rz};
     store_partial<1>(a.part, v);
-    if (last_block(&a.st->ticket[TICKET_AUX])) {
+    if (last_block(&a.st->ticket)) {
         double t[1];
         grid_total<1>(a.part, gridDim.x, t);
         if (threadIdx.x == 0) {
-            a.st->ticket[TICKET_AUX] = 0;
+            a.st->ticket = 0;
             a.st->rz = t[0];
         }
     }
@@ -1392,11 +1473,11 @@ __global__ void __launch_bounds__(kNodeBS) k_refresh_residual(NodeArgs<float> a)
     }
     double v[1] = {rr};
     store_partial<1>(a.part, v);
-    if (last_block(&st->ticket[TICKET_AUX])) {
+    if (last_block(&st->ticket)) {
         double t[1];
         grid_total<1>(a.part, gridDim.x, t);
         if (threadIdx.x == 0) {
-            st->ticket[TICKET_AUX] = 0;
+            st->ticket = 0;
             const double s_new = sqrt(t[0]);
             st->alpha = 0.0;  // the last step is in x64 now (k_refresh_flush)
             st->nupd += 1;
@@ -1409,20 +1490,6 @@ __global__ void __launch_bounds__(kNodeBS) k_refresh_residual(NodeArgs<float> a)
             }
         }
     }
-}
-
-// Sum over the warp of lanes' slot counts before this lane: the exclusive prefix
-// that, added to hbase[node / 32], gives the node's first halo slot. Every lane of
-// the warp calls it; the warp's lanes hold 32 consecutive nodes from a multiple of
-// 32 (lanes past the end pass cnt = 0).
-__device__ __forceinline__ int halo_prefix(int cnt, int lane) {
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-    }
-    return incl - cnt;
 }
 
 // MIXED refresh 3, halo mode: as k_refresh_residual, with K x64 on free rows =
@@ -1458,11 +1525,11 @@ __global__ void __launch_bounds__(kNodeBS) k_refresh_residual_halo(NodeArgs<floa
     }
     double v[1] = {rr};
     store_partial<1>(a.part, v);
-    if (last_block(&st->ticket[TICKET_AUX])) {
+    if (last_block(&st->ticket)) {
         double t[1];
         grid_total<1>(a.part, gridDim.x, t);
         if (threadIdx.x == 0) {
-            st->ticket[TICKET_AUX] = 0;
+            st->ticket = 0;
             const double s_new = sqrt(t[0]);
             st->alpha = 0.0;  // the last step is in x64 now (k_refresh_flush)
             st->nupd += 1;
@@ -1530,11 +1597,11 @@ __global__ void __launch_bounds__(kNodeBS) k_refresh_rescale(NodeArgs<float> a) 
     }
     double v[1] = {rz};
     store_partial<1>(a.part, v);
-    if (last_block(&st->ticket[TICKET_AUX])) {
+    if (last_block(&st->ticket)) {
         double t[1];
         grid_total<1>(a.part, gridDim.x, t);
         if (threadIdx.x == 0) {
-            st->ticket[TICKET_AUX] = 0;
+            st->ticket = 0;
             const double ratio2 = st->ratio * st->ratio;
             st->beta = t[0] / (st->rz_old * ratio2);
             st->rz = t[0];

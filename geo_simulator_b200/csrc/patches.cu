@@ -239,10 +239,10 @@ __global__ void k_local_conn(const int32_t* __restrict__ conn, const int32_t* __
     const int l = (int)(t % 10);
     const int32_t nn = ninv[conn[l * E + eperm[ne]]];
     const int p = (int)(ne / kPatchElems);
-    const int32_t own0 = po[p], nown = po[p + 1] - own0;
+    const int32_t own0 = po[p], base = patch_align(own0), nown = po[p + 1] - base;
     int64_t loc;
     if (nn >= own0) {
-        loc = nn - own0;
+        loc = nn - base;
         if (loc >= nown) atomicOr(err, DEV_ERR_BOUNDS);
     } else {
         int64_t lo = pf[p], hi = pf[p + 1];
@@ -254,15 +254,14 @@ __global__ void k_local_conn(const int32_t* __restrict__ conn, const int32_t* __
         if (lo >= pf[p + 1] || foreign[lo] != nn) atomicOr(err, DEV_ERR_BOUNDS);
         loc = nown + (lo - pf[p]);
     }
-    const int64_t slot = loc + (loc >> 5);  // patch_slot
-    if (slot > 65535) atomicOr(err, DEV_ERR_BOUNDS);
-    lconn[(int64_t)l * E + ne] = (uint16_t)slot;
+    if (4 * patch_slot32((int)loc) > 65535) atomicOr(err, DEV_ERR_BOUNDS);
+    lconn[(int64_t)l * E + ne] = (uint16_t)patch_slot((int)loc);
 }
 
 __global__ void k_local_sizes(const int32_t* po, const int32_t* pf, int P, int* out) {
     int m = 0;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x)
-        m = max(m, (po[p + 1] - po[p]) + (pf[p + 1] - pf[p]));
+        m = max(m, (po[p + 1] - patch_align(po[p])) + (pf[p + 1] - pf[p]));
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
@@ -279,7 +278,7 @@ __global__ void __launch_bounds__(32 * kOrderWarps)
 k_patch_order(const uint16_t* __restrict__ lconn, int64_t E, const int32_t* __restrict__ pe, int P,
               int32_t* __restrict__ wperm) {
     __shared__ uint16_t sl[kOrderWarps][10][kPatchElems];
-    __shared__ uint32_t used[kOrderWarps][(patch_slot(10 * kPatchElems) + 31) / 32];
+    __shared__ uint32_t used[kOrderWarps][(patch_slot(10 * kPatchElems + kNodeAlign) + 31) / 32];
     __shared__ uint8_t taken[kOrderWarps][kPatchElems];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int p = blockIdx.x * kOrderWarps + w;
@@ -349,10 +348,12 @@ k_patch_order(const uint16_t* __restrict__ lconn, int64_t E, const int32_t* __re
 }
 
 // Applies the within-patch order: eperm2[ne] = eperm[wperm[ne]] and the
-// patch-major paired connectivity (see PatchLayout::lc).
+// patch-major paired connectivity (see PatchLayout::lc and lc32).
 __global__ void k_apply_order(const int32_t* __restrict__ wperm, const int32_t* __restrict__ eperm,
                               const uint16_t* __restrict__ lconn, int64_t E, int P, int32_t* __restrict__ eperm2,
-                              uint32_t* __restrict__ lc) {
+                              uint32_t* __restrict__ lc, uint32_t* __restrict__ lc32) {
+    // slot u + u/32 -> 4 (u + 34 (u/32)): every row of 33 slots becomes one of 66
+    auto slot32 = [](uint32_t s) { return 4u * (s + 33u * (s / 33u)); };
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= (int64_t)P * kPatchElems) return;
     const int64_t p = t / kPatchElems, j = t % kPatchElems;
@@ -360,11 +361,13 @@ __global__ void k_apply_order(const int32_t* __restrict__ wperm, const int32_t* 
     if (ne < E) {
         const int64_t src = wperm[ne];
         eperm2[ne] = eperm[src];
-        for (int l2 = 0; l2 < 5; ++l2)
-            lc[(p * 5 + l2) * kPatchElems + j] =
-                (uint32_t)lconn[(int64_t)(2 * l2) * E + src] | (uint32_t)lconn[(int64_t)(2 * l2 + 1) * E + src] << 16;
+        for (int l2 = 0; l2 < 5; ++l2) {
+            const uint32_t a = lconn[(int64_t)(2 * l2) * E + src], b = lconn[(int64_t)(2 * l2 + 1) * E + src];
+            lc[(p * 5 + l2) * kPatchElems + j] = a | b << 16;
+            lc32[(p * 5 + l2) * kPatchElems + j] = slot32(a) | slot32(b) << 16;
+        }
     } else {
-        for (int l2 = 0; l2 < 5; ++l2) lc[(p * 5 + l2) * kPatchElems + j] = 0u;
+        for (int l2 = 0; l2 < 5; ++l2) lc[(p * 5 + l2) * kPatchElems + j] = lc32[(p * 5 + l2) * kPatchElems + j] = 0u;
     }
 }
 
@@ -465,8 +468,9 @@ void build_patches(cudaStream_t s, int64_t N, const double* xyz, int64_t E, cons
         k_patch_order<<<(unsigned)cdiv(P, kOrderWarps), 32 * kOrderWarps, 0, s>>>(lconn.p, E, L.patch_elem.p, P,
                                                                                   wperm.p);
         L.lc.alloc((size_t)P * 5 * kPatchElems);
+        L.lc32.alloc((size_t)P * 5 * kPatchElems);
         k_apply_order<<<nb((int64_t)P * kPatchElems), 256, 0, s>>>(wperm.p, L.eperm.p, lconn.p, E, P, eperm2.p,
-                                                                    L.lc.p);
+                                                                    L.lc.p, L.lc32.p);
         GEO_CUDA(cudaGetLastError());
         GEO_CUDA(cudaStreamSynchronize(s));
         L.eperm = std::move(eperm2);

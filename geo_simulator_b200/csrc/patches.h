@@ -24,6 +24,17 @@ constexpr int kPatchElems = 384;
 // 2.8 shared-memory wavefronts per warp access of the element phase). The 16-bit
 // local connectivity holds slots; loops over a patch's nodes map u -> slot.
 __host__ __device__ constexpr int patch_slot(int u) { return u + (u >> 5); }
+// The same node in the FP32 kernels' table, whose rows of 32 nodes (33 slots) hold the
+// node values and then the accumulators of the same nodes: both at a constant distance,
+// so one address serves the element gather and the scatter. The FP32 connectivity
+// holds 4 * patch_slot32 (a byte offset for one DOF per node).
+__host__ __device__ constexpr int patch_slot32(int u) { return u + 34 * (u >> 5); }
+
+// Patch-local numbering: own node j (global patch numbering) is local j - align(o0),
+// so that aligned groups of kNodeAlign consecutive nodes are groups in both numberings
+// and a thread can move one with 16-byte accesses; foreign nodes follow the own range.
+constexpr int kNodeAlign = 4;
+__host__ __device__ constexpr int patch_align(int o0) { return o0 & ~(kNodeAlign - 1); }
 
 // node flag bits (patch numbering)
 constexpr uint8_t kFlagDir0 = 1;      // component c is Dirichlet: kFlagDir0 << c
@@ -46,6 +57,7 @@ struct PatchLayout {
     // past a short last patch are 0). Within a patch, elements are ordered so that
     // every aligned group of 32 (one warp) shares no node where possible.
     DevBuf<uint32_t> lc;            // [n_patches][5][kPatchElems]
+    DevBuf<uint32_t> lc32;          // the same with 4 * patch_slot32 for the FP32 kernels
     DevBuf<uint8_t> shared;         // [n_nodes] patch numbering: 1 if shared
 };
 
