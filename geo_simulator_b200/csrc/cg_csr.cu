@@ -5,7 +5,7 @@
 // One persistent cooperative kernel runs the whole solve: sub-warp SpMV,
 // Jacobi scaling, axpys, and dot products reduced by warp shuffles into
 // per-block partials that every block sums in the same fixed order after a
-// bounded grid barrier (so all blocks take identical, deterministic decisions).
+// bounded grid-wide wait (so all blocks take identical, deterministic decisions).
 #include <mutex>
 
 #include "pcg_common.cuh"
@@ -13,7 +13,8 @@
 namespace geo {
 namespace {
 
-constexpr int kBS = 256;
+constexpr int kBS = 256;     // threads of a block
+constexpr int kBSOne = 1024;  // most threads of a block when the rows take one pass of the grid
 #ifndef GEO_CSR_VEC
 #define GEO_CSR_VEC 4
 #endif
@@ -36,6 +37,7 @@ struct CsrPcgArgs {
     const double* b;
     double *x, *r, *p, *q, *dinv;
     double *part_a, *part_b;
+    GridSlot* slots;  // [2][2][blocks], zero before the launch (ONE_PASS)
     GridSync* gs;
     PcgResult* res;
     unsigned long long timeout_ns;
@@ -53,15 +55,34 @@ __device__ __forceinline__ int64_t lower_bound_i32(const int32_t* idx, int64_t b
     return b;
 }
 
-__global__ void __launch_bounds__(kBS, 4) k_csr_pcg(CsrPcgArgs a) {
+// ONE_PASS (n <= 256 rows per SM, pcg_grid): one block per SM and grid-wide exchanges in
+// place of barrier and partial sums: such a system spends its iterations on them (2197
+// rows: 19.3 -> 10.3 us per iteration, 35,937 rows 23.0 -> 20.3). Larger systems keep four
+// blocks of 256 threads per SM, which the SpMV's loads overlap better (402,675 rows: 54.6
+// us, 59.3 before the barrier lost two fences and the partials a serial sum, against 60
+// with one block per SM and exchanges). Streaming the matrix through shared memory was
+// slower (71 us): it takes the L1 that holds the gathered p.
+template <bool ONE_PASS>
+__global__ void __launch_bounds__(ONE_PASS ? kBSOne : kBS, ONE_PASS ? 1 : 4) k_csr_pcg(CsrPcgArgs a) {
     const unsigned nb = gridDim.x;
+    unsigned long long turn = 0;
+    // sums v over the grid, valid everywhere; a grid-wide barrier at the same time
+    auto all_sum = [&](auto& v, double* part) {
+        constexpr int K = sizeof(v) / sizeof(double);
+        if (ONE_PASS) return grid_all_sum<K>(a.slots, 2 * (int)nb, a.gs, (int)nb, turn, a.timeout_ns, v);
+        store_partial<K>(part, v);
+        if (!grid_barrier(a.gs, nb, a.timeout_ns)) return false;
+        grid_total<K>(part, nb, v);
+        return true;
+    };
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t nth = (int64_t)gridDim.x * blockDim.x;
     const int64_t n = a.n;
 
     // x = 0, r = b, z = M^-1 r, p = z (iterative.rs:70-75)
+    double t2[2] = {0.0, 0.0};
     {
-        double v[2] = {0.0, 0.0};
+        double (&v)[2] = t2;
         for (int64_t i = tid; i < n; i += nth) {
             double di = 1.0;
             if (a.use_prec) {
@@ -81,11 +102,8 @@ __global__ void __launch_bounds__(kBS, 4) k_csr_pcg(CsrPcgArgs a) {
             v[0] += bi * bi;
             v[1] += bi * zi;
         }
-        store_partial<2>(a.part_b, v);
     }
-    if (!grid_barrier(a.gs, nb, a.timeout_ns)) return;
-    double t2[2];
-    grid_total<2>(a.part_b, nb, t2);
+    if (!all_sum(t2, a.part_b)) return;
     const double bnorm = sqrt(t2[0]);
     double rz = t2[1];
     if (bnorm < 1e-25) {  // iterative.rs:60-68
@@ -100,8 +118,9 @@ __global__ void __launch_bounds__(kBS, 4) k_csr_pcg(CsrPcgArgs a) {
     constexpr int rows_per_warp = 32 / kVec;
     while (it < a.max_it) {
         // q = A p and p.q
+        double pq[1] = {0.0};
         {
-            double v[1] = {0.0};
+            double (&v)[1] = pq;
             for (int64_t rbase = warp * rows_per_warp; rbase < n; rbase += nwarps * rows_per_warp) {
                 const int64_t row = rbase + lane / kVec;
                 double s = 0.0;
@@ -132,18 +151,16 @@ __global__ void __launch_bounds__(kBS, 4) k_csr_pcg(CsrPcgArgs a) {
                     v[0] += a.p[row] * s;
                 }
             }
-            store_partial<1>(a.part_a, v);
         }
-        if (!grid_barrier(a.gs, nb, a.timeout_ns)) return;
-        double pq[1];
-        grid_total<1>(a.part_a, nb, pq);
+        if (!all_sum(pq, a.part_a)) return;
         if (fabs(pq[0]) < 1e-30) {  // iterative.rs:85
             breakdown = 1;
             break;
         }
         const double alpha = rz / pq[0];
+        t2[0] = t2[1] = 0.0;
         {
-            double v[2] = {0.0, 0.0};
+            double (&v)[2] = t2;
             for (int64_t i = tid; i < n; i += nth) {
                 const double pi = a.p[i];
                 a.x[i] += alpha * pi;
@@ -152,10 +169,8 @@ __global__ void __launch_bounds__(kBS, 4) k_csr_pcg(CsrPcgArgs a) {
                 v[0] += ri * ri;
                 v[1] += ri * (ri * a.dinv[i]);
             }
-            store_partial<2>(a.part_b, v);
         }
-        if (!grid_barrier(a.gs, nb, a.timeout_ns)) return;
-        grid_total<2>(a.part_b, nb, t2);
+        if (!all_sum(t2, a.part_b)) return;
         const double rn = sqrt(t2[0]);
         final_res = rn;
         if (rn < a.tol * bnorm || rn < a.abs_tol) {  // iterative.rs:95
@@ -165,10 +180,38 @@ __global__ void __launch_bounds__(kBS, 4) k_csr_pcg(CsrPcgArgs a) {
         const double beta = t2[1] / rz;
         rz = t2[1];
         for (int64_t i = tid; i < n; i += nth) a.p[i] = a.r[i] * a.dinv[i] + beta * a.p[i];
-        if (!grid_barrier(a.gs, nb, a.timeout_ns)) return;
+        if (ONE_PASS) {
+            double none[1] = {0.0};
+            if (!all_sum(none, nullptr)) return;
+        } else {
+            if (!grid_barrier(a.gs, nb, a.timeout_ns)) return;
+        }
         ++it;
     }
     if (tid == 0) *a.res = PcgResult{it, final_res, bnorm, converged, breakdown, 0};
+}
+
+// Form and grid of the persistent kernel. Systems of at most 256 rows (kVec lanes each of
+// a 1024-thread block) per SM take one block per SM, of 256 threads where that still holds
+// all rows (cheaper block barriers), and fewer blocks where they have fewer rows.
+struct PcgGrid {
+    int nb, bs;
+    bool one_pass;
+};
+PcgGrid pcg_grid(geo_ctx* ctx, int64_t n) {
+    const int one = persistent_blocks(ctx, k_csr_pcg<true>, kBSOne, 0);
+    if (n * kVec > (int64_t)one * kBSOne) return {persistent_blocks(ctx, k_csr_pcg<false>, kBS, 0), kBS, false};
+    int bs = 256;
+    while (bs < kBSOne && n * kVec > (int64_t)one * bs) bs *= 2;
+    return {(int)std::max<int64_t>(1, std::min<int64_t>(one, cdiv(n * kVec, bs))), bs, true};
+}
+void launch_pcg(geo_ctx* ctx, CsrPcgArgs& args, const PcgGrid& g) {
+    if (g.one_pass) {
+        GEO_CUDA(cudaMemsetAsync(args.slots, 0, (size_t)g.nb * 4 * sizeof(GridSlot), ctx->stream));
+        launch_persistent(ctx, k_csr_pcg<true>, g.bs, 0, args, g.nb);
+    } else {
+        launch_persistent(ctx, k_csr_pcg<false>, g.bs, 0, args, g.nb);
+    }
 }
 
 }  // namespace
@@ -201,7 +244,8 @@ int geo_cg_solve(geo_ctx* ctx, const geo_csr* A, const double* b, const geo_cg_o
     const int64_t n = A->n_rows;
     DevBuf<double> tb, work(5 * n);
     const double* db = stage_in(b, n, tb, s);
-    const int nb = persistent_blocks(ctx, k_csr_pcg, kBS, 0);
+    const PcgGrid grid = pcg_grid(ctx, n);
+    const int nb = grid.nb;
     PcgScratch sc;
     sc.ensure(nb);
     CsrPcgArgs args{};
@@ -217,6 +261,7 @@ int geo_cg_solve(geo_ctx* ctx, const geo_csr* A, const double* b, const geo_cg_o
     args.dinv = work.p + 4 * n;
     args.part_a = sc.slot(0, nb);
     args.part_b = sc.slot(1, nb);
+    args.slots = reinterpret_cast<GridSlot*>(sc.part.p);  // 3 x 4 doubles per block: room for 4 slots
     args.gs = sc.gs.p;
     args.res = sc.res.p;
     args.timeout_ns = (unsigned long long)(o.timeout_seconds * 1e9);
@@ -227,7 +272,7 @@ int geo_cg_solve(geo_ctx* ctx, const geo_csr* A, const double* b, const geo_cg_o
     GEO_CUDA(cudaMemsetAsync(sc.gs.p, 0, sizeof(GridSync), s));
     GEO_CUDA(cudaMemsetAsync(sc.res.p, 0, sizeof(PcgResult), s));
     GEO_CUDA(cudaEventRecord(ctx->ev0, s));
-    launch_persistent(ctx, k_csr_pcg, kBS, 0, args, nb);
+    launch_pcg(ctx, args, grid);
     GEO_CUDA(cudaEventRecord(ctx->ev1, s));
     PcgResult r{};
     GridSync g{};
@@ -374,7 +419,8 @@ extern "C" int geo_cg_solve_noalloc(geo_ctx* ctx, const geo_csr* A, const double
     geo_cg_opts o;
     cg_opts_fill(opts, o);
     GEO_CHECK_ARG(o.max_iterations >= 0, "max_iterations must be >= 0");
-    const int nb = persistent_blocks(ctx, k_csr_pcg, kBS, 0);
+    const PcgGrid grid = pcg_grid(ctx, n);
+    const int nb = grid.nb;
     if (nb > kNoAllocMaxBlocks) fail(GEO_ERR_UNSUPPORTED, "geo_cg_solve_noalloc: persistent grid too large");
     cudaStream_t s = ctx->stream;
     double* vec = reinterpret_cast<double*>(base);
@@ -393,6 +439,7 @@ extern "C" int geo_cg_solve_noalloc(geo_ctx* ctx, const geo_csr* A, const double
     args.dinv = vec + 3 * (size_t)GEO_NOALLOC_MAX_ROWS;
     args.part_a = reinterpret_cast<double*>(base + kNoAllocOffPart);
     args.part_b = reinterpret_cast<double*>(base + kNoAllocOffPart + kNoAllocPartBytes);
+    args.slots = reinterpret_cast<GridSlot*>(base + kNoAllocOffPart);  // both partial areas: 8 doubles per block
     args.gs = gs;
     args.res = res;
     args.timeout_ns = (unsigned long long)(o.timeout_seconds * 1e9);
@@ -403,7 +450,7 @@ extern "C" int geo_cg_solve_noalloc(geo_ctx* ctx, const geo_csr* A, const double
     GEO_CUDA(cudaMemsetAsync(gs, 0, sizeof(GridSync), s));
     GEO_CUDA(cudaMemsetAsync(res, 0, sizeof(PcgResult), s));
     GEO_CUDA(cudaEventRecord(ctx->ev0, s));
-    launch_persistent(ctx, k_csr_pcg, kBS, 0, args, nb);
+    launch_pcg(ctx, args, grid);
     GEO_CUDA(cudaEventRecord(ctx->ev1, s));
     PcgResult r{};
     GridSync g{};

@@ -166,8 +166,9 @@ __device__ __forceinline__ bool grid_barrier(GridSync* gs, unsigned int nblocks,
         cuda::atomic_ref<unsigned int, cuda::thread_scope_device> cnt(gs->count);
         cuda::atomic_ref<int, cuda::thread_scope_device> err(gs->error);
         int ok = 1;
-        const unsigned int g = gen.load(cuda::memory_order_acquire);
-        __threadfence();
+        // thread 0's release (the arrival) and acquire (the new generation) cover the block's
+        // other threads through the block barriers on either side
+        const unsigned int g = gen.load(cuda::memory_order_relaxed);
         if (cnt.fetch_add(1u, cuda::memory_order_acq_rel) == nblocks - 1) {
             cnt.store(0u, cuda::memory_order_relaxed);
             gen.fetch_add(1u, cuda::memory_order_release);
@@ -187,7 +188,6 @@ __device__ __forceinline__ bool grid_barrier(GridSync* gs, unsigned int nblocks,
             }
         }
         if (ok && err.load(cuda::memory_order_relaxed) != 0) ok = 0;
-        __threadfence();
         s_ok = ok;
     }
     __syncthreads();
@@ -255,6 +255,110 @@ __device__ __forceinline__ void grid_total(const double* part, int nblocks, doub
 #pragma unroll
     for (int k = 0; k < K; ++k) out[k] = tot[k];
     __syncthreads();
+}
+
+// A block's contribution to grid_all_sum: value and epoch, written and read as one word.
+struct __align__(16) GridSlot {
+    double v;
+    unsigned long long epoch;
+};
+__device__ __forceinline__ void slot_put(GridSlot* s, double v, unsigned long long epoch) {
+    asm volatile("{\n .reg .b128 q;\n mov.b128 q, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], q;\n}\n"
+                 :: "l"(s), "l"(__double_as_longlong(v)), "l"(epoch) : "memory");
+}
+__device__ __forceinline__ unsigned long long slot_get(const GridSlot* s, double& v) {
+    unsigned long long lo, hi;
+    asm volatile("{\n .reg .b128 q;\n ld.relaxed.gpu.global.b128 q, [%2];\n mov.b128 {%0, %1}, q;\n}\n"
+                 : "=l"(lo), "=l"(hi) : "l"(s) : "memory");
+    v = __longlong_as_double((long long)lo);
+    return hi;
+}
+
+// Grid-wide barrier and sum in one exchange, for a co-resident grid: every block publishes
+// its K sums with the running number of the exchange, and its first warp waits for those
+// of all blocks and adds them in a fixed order (bit-identical totals everywhere, valid in
+// all threads). Against grid_barrier and grid_total it saves the counter that all blocks
+// queue at, the wait for its generation, the load of the partials behind it and three of
+// five block barriers. slots: [2][stride], stride >= K nblocks, all of it zero before the
+// launch; turn counts the exchanges of the kernel and starts at 0. A block reuses a slot
+// two exchanges later, when every block has read it. Bounded as grid_barrier; false on
+// timeout.
+template <int K>
+__device__ __forceinline__ bool grid_all_sum(GridSlot* slots, int stride, GridSync* gs, int nblocks,
+                                             unsigned long long& turn, unsigned long long timeout_ns, double (&v)[K]) {
+    __shared__ double red[2][32][K], tot[2][K];
+    __shared__ int s_ok[2];
+    const int par = (int)(turn & 1), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    GridSlot* mine = slots + par * stride;
+    ++turn;
+    auto warp_sum = [&]() {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+    };
+    warp_sum();
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < K; ++k) red[par][warp][k] = v[k];
+    __syncthreads();  // puts the block's work before the release below
+    if (warp == 0) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] = lane < (int)(blockDim.x >> 5) ? red[par][lane][k] : 0.0;
+        warp_sum();
+        if (lane == 0) {
+            cuda::atomic_thread_fence(cuda::memory_order_release, cuda::thread_scope_device);
+#pragma unroll
+            for (int k = 0; k < K; ++k) slot_put(mine + k * nblocks + blockIdx.x, v[k], turn);
+        }
+        bool ok = true;
+        unsigned long long t0 = 0;
+        unsigned int spins = 0;
+        cuda::atomic_ref<int, cuda::thread_scope_device> err(gs->error);
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] = 0.0;
+        constexpr int kFlight = 5;  // slots per lane and sum in flight: 160 blocks at a time
+        for (int b0 = lane; b0 < nblocks && ok; b0 += 32 * kFlight) {
+            double w[kFlight][K];
+            bool all;
+            do {
+                all = true;
+#pragma unroll
+                for (int i = 0; i < kFlight; ++i)
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        const int b = b0 + 32 * i;
+                        w[i][k] = 0.0;
+                        if (b < nblocks && slot_get(mine + k * nblocks + b, w[i][k]) != turn) all = false;
+                    }
+                if (!all && (++spins & 15u) == 0) {
+                    const unsigned long long now = global_timer_ns();
+                    if (t0 == 0) t0 = now;
+                    if (err.load(cuda::memory_order_relaxed) != 0) ok = false;
+                    if (now - t0 > timeout_ns) {
+                        err.fetch_or(DEV_ERR_TIMEOUT, cuda::memory_order_relaxed);
+                        ok = false;
+                    }
+                }
+            } while (!all && ok);
+#pragma unroll
+            for (int i = 0; i < kFlight; ++i)
+#pragma unroll
+                for (int k = 0; k < K; ++k) v[k] += w[i][k];
+        }
+        cuda::atomic_thread_fence(cuda::memory_order_acquire, cuda::thread_scope_device);
+        ok = __all_sync(0xffffffffu, ok);
+        warp_sum();
+        if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) tot[par][k] = v[k];
+            s_ok[par] = ok;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = tot[par][k];
+    return s_ok[par] != 0;
 }
 
 // Block-level partial of K doubles -> part[blockIdx.x*K + k] (thread 0 writes).
