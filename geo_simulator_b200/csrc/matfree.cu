@@ -644,15 +644,44 @@ int setup_patch_kernels(geo_op* op, int slot) {
     return per_sm * op->ctx->sm_count;
 }
 
+// The PCG loop's kernels use programmatic dependent launch up to this many dofs: the next
+// kernel's blocks then start on the SMs that the last blocks of the one before leave, and
+// set up shared memory and the first patch's element copies before they wait. Per
+// iteration, without and with: 6^3 FP64 12.5 -> 11.6 us, 16^3 mixed 16.8 -> 15.1,
+// 48x48x32 mixed 24.1 -> 23.5, 64^3 FP64 (2.1 M dofs) 95.1 -> 92.6, elastic 48x48x24 mixed
+// (1.4 M) 41.5 -> 40.8. With more there is nothing to gain (elastic 48^3, 2.7 M: 169.8,
+// 169.7), and the mixed solver loses (thermal 80^3, 4.2 M: 96.7 -> 98.4; 128^3: 330 -> 342).
+constexpr int64_t kDependentDofs = 2500000;
+
+// Launches k, with programmatic dependent launch when `dependent`: its blocks may start, up
+// to their griddepcontrol.wait, while the kernel before it in the stream still runs. Only
+// for kernels of a captured chunk: k_patch reads the operator's element data before its
+// wait, which must not be the output of the kernel before it.
+template <class... P, class... A>
+void launch_dependent(bool dependent, void (*k)(P...), unsigned grid, int bs, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(bs);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = dependent ? 1 : 0;
+    GEO_CUDA(cudaLaunchKernelEx(&cfg, k, P(args)...));
+}
+
 // Blocks of the patch kernel: the resident ones, or one per patch.
 unsigned patch_blocks(const geo_op* op, int slot) { return (unsigned)std::min(op->patch_grid[slot], op->n_patches); }
 
 template <class K, class T, int MODE>
-void launch_patch(const geo_op* op, int slot, cudaStream_t s, const T* qd, const PatchArgs<T>& pa) {
+void launch_patch(const geo_op* op, int slot, cudaStream_t s, const T* qd, const PatchArgs<T>& pa, bool dependent = false) {
     PatchView v = view(op);
     v.own_bulk = op->own_bulk[slot];
     with_patch_kernel<K, T, MODE>(op->nbuf[slot], op->halo[slot], [&](auto k) {
-        k<<<patch_blocks(op, slot), kPatchBS, op->patch_smem[slot], s>>>(v, qd, (T)op->cl, (T)op->cm, pa);
+        launch_dependent(dependent, k, patch_blocks(op, slot), kPatchBS, op->patch_smem[slot], s, v, qd,
+                         (T)op->cl, (T)op->cm, pa);
     });
 }
 
@@ -981,20 +1010,21 @@ unsigned update_blocks(const geo_op* op, int slot) {
 // The node update of the PCG loop: the halo-mode kernel when the patch kernel runs
 // in halo mode.
 template <class K, class T, bool MIXED>
-void launch_update(const geo_op* op, cudaStream_t s, const NodeArgs<T>& na) {
+void launch_update(const geo_op* op, cudaStream_t s, const NodeArgs<T>& na, bool dependent = false) {
     constexpr int slot = std::is_same<T, double>::value ? 0 : 1;
     const unsigned g = update_blocks(op, slot);
-    if (op->halo[slot]) k_pcg_update_halo<T, K::DPN, MIXED><<<g, kNodeBS, 0, s>>>(na);
-    else k_pcg_update<T, K::DPN, MIXED><<<g, kNodeBS, 0, s>>>(na);
+    launch_dependent(dependent, op->halo[slot] ? k_pcg_update_halo<T, K::DPN, MIXED> : k_pcg_update<T, K::DPN, MIXED>, g,
+                     kNodeBS, 0, s, na);
 }
 
-// Enqueues one PCG iteration (patch kernel in PCG mode + node update).
+// Enqueues one PCG iteration (patch kernel in PCG mode + node update) of a captured chunk.
 template <class K, class T, bool MIXED>
 void enqueue_iteration(geo_op* op, cudaStream_t s, const PatchArgs<T>& pa, const NodeArgs<T>& na) {
     constexpr bool dbl = std::is_same<T, double>::value;
     const T* qd = dbl ? (const T*)op->qd64.p : (const T*)op->qd32.p;
-    launch_patch<K, T, MODE_PCG>(op, dbl ? 0 : 1, s, qd, pa);
-    launch_update<K, T, MIXED>(op, s, na);
+    const bool dependent = op->ndof <= kDependentDofs;
+    launch_patch<K, T, MODE_PCG>(op, dbl ? 0 : 1, s, qd, pa, dependent);
+    launch_update<K, T, MIXED>(op, s, na, dependent);
 }
 
 // Kernel arguments of the PCG loop over the operator's workspace (FP64 mode: r, q,
