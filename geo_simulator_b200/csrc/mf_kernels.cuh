@@ -38,10 +38,11 @@
 // scalars, state store, then the next kernel's load of the state) put 3 to 4 us of
 // dependent latency behind each of the two kernels: with the folds an iteration takes
 // 13.0 instead of 19.0 us at 6^3 (FP64), 23.9 instead of 33.4 us at 48x48x32 (mixed)
-// and 24.1 instead of 31.0 us for FP64 elasticity at 27x22x13. Two copies of PcgState alternate, so that block 0 never
-// writes the copy that other blocks of its grid still read. The kernels outside the
-// loop (start, refresh) keep the ticket form. No host round trip per iteration and
-// no grid-wide spin wait.
+// and 24.1 instead of 31.0 us for FP64 elasticity at 27x22x13. Two copies of PcgState
+// alternate, so that block 0 never writes the copy that other blocks of its grid still
+// read. The kernels outside the loop (start, refresh) keep the ticket form. The loop is
+// one CUDA graph that the device steers (build_loop): no host round trip within a solve
+// and no grid-wide spin wait.
 #pragma once
 
 #include <type_traits>
@@ -232,11 +233,13 @@ struct PcgScalars {
     int flags;
     int pending;  // the node update's partials (r.r, r.z) are not folded in yet
 };
-// With the words that the kernels of the loop do not copy along: the DEV_ERR_* bits
-// raised by bounded waits and the ticket counter (first copy only).
+// With the words that the kernels of the loop do not copy along (first copy only): the
+// DEV_ERR_* bits raised by bounded waits, the ticket counter, and the chunks run and
+// allowed.
 struct PcgState : PcgScalars {
     int err;
     unsigned int ticket;
+    long long chunks, max_chunks;
 };
 
 template <class T>
@@ -390,13 +393,22 @@ __device__ __forceinline__ PcgHead pcg_fold(const PcgState* in, PcgState* out,
     return PcgHead{s_st.alpha, s_st.beta, s_st.cd, (int)(s_st.it & 1), s_st.flags};
 }
 
-// End of a chunk of iterations: folds the last node update's partials in, so that the
-// host reads a decided state. One block.
+// End of a chunk of iterations: folds the last node update's partials in and decides
+// whether the graph's loop runs another chunk (`again`) and whether the refresh comes
+// first (`refresh`, mixed). One block.
 template <bool MIXED>
-__global__ void __launch_bounds__(kNodeBS) k_pcg_decide(PcgState* st, const double* __restrict__ part, int n) {
-    pcg_fold(st, st, part, n, [](PcgScalars& s, double t0, double t1) {
+__global__ void __launch_bounds__(kNodeBS) k_pcg_decide(PcgState* st, const double* __restrict__ part, int n,
+                                                        cudaGraphConditionalHandle again,
+                                                        cudaGraphConditionalHandle refresh) {
+    const PcgHead h = pcg_fold(st, st, part, n, [](PcgScalars& s, double t0, double t1) {
         if (s.pending) pcg_next_iteration<MIXED>(s, t0, t1);
     });
+    if (threadIdx.x == 0) {
+        const long long chunks = ++st->chunks;
+        const bool stop = (h.flags & ST_DONE) || st->err || chunks >= st->max_chunks;
+        cudaGraphSetConditional(again, stop ? 0u : 1u);
+        if (MIXED) cudaGraphSetConditional(refresh, !stop && (h.flags & ST_REFRESH) ? 1u : 0u);
+    }
 }
 
 // bytes of one patch's element data (connectivity + qdata), 16-byte multiple
@@ -1006,6 +1018,7 @@ struct NodeArgs {
     const T* halo;
     const int32_t* hbase;
     const double* halo64;  // mixed refresh: FP64 slots of the FP64 apply (halo mode)
+    cudaGraphConditionalHandle again;  // mixed refresh: cleared when it ends the solve
 };
 
 constexpr int kHaloShift = 3;  // flag bits 3-6: halo slots of the node (halo mode)
@@ -1505,6 +1518,7 @@ __global__ void __launch_bounds__(kNodeBS) k_refresh_residual(NodeArgs<float> a)
             st->s_new = s_new;
             if (s_new < st->tol * st->bnorm || s_new < st->abs_tol) {
                 st->flags = (st->flags & ~ST_REFRESH) | ST_DONE | ST_CONVERGED;
+                cudaGraphSetConditional(a.again, 0u);
             } else {
                 st->ratio = st->s_scale / s_new;
             }
@@ -1557,6 +1571,7 @@ __global__ void __launch_bounds__(kNodeBS) k_refresh_residual_halo(NodeArgs<floa
             st->s_new = s_new;
             if (s_new < st->tol * st->bnorm || s_new < st->abs_tol) {
                 st->flags = (st->flags & ~ST_REFRESH) | ST_DONE | ST_CONVERGED;
+                cudaGraphSetConditional(a.again, 0u);
             } else {
                 st->ratio = st->s_scale / s_new;
             }
@@ -1628,7 +1643,10 @@ __global__ void __launch_bounds__(kNodeBS) k_refresh_rescale(NodeArgs<float> a) 
             st->s_scale = st->s_new;
             st->rmax = 1.0;
             st->flags &= ~ST_REFRESH;
-            if (st->it >= st->max_it) st->flags |= ST_DONE;
+            if (st->it >= st->max_it) {
+                st->flags |= ST_DONE;
+                cudaGraphSetConditional(a.again, 0u);
+            }
         }
     }
 }

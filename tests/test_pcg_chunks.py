@@ -1,6 +1,7 @@
 """The PCG loop's launch forms: kernels started before the one before them has ended (up to
 2.5 M dofs), and not (above). A solution's residual, formed by the operator apply, meets
-the tolerance that the solver says it met."""
+the tolerance that the solver says it met. And the iteration limit inside, at the end and
+behind the end of a pass of the loop."""
 import numpy as np
 import pytest
 
@@ -36,3 +37,22 @@ def test_residual_of_solution(orc, geo, physics, shape, precision):
     # and the same bits again: every sum has a fixed order
     x2, st2 = op.solve(fb, solver)
     assert st2.iterations == st.iterations and np.array_equal(x, x2)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("limit", [1, 15, 16, 17, 33])
+def test_iteration_limit(orc, geo, limit, precision):
+    box = (1000.0, 1000.0, 600.0)
+    xyz, conn = orc.generate_cube(6, 6, 6, *box)
+    mask, vals = orc.thermal_bc(xyz, box[2])
+    dm = geo.DofManager(xyz.shape[0], 1)
+    idx = np.nonzero(mask)[0]
+    dm.set_dirichlet(idx, vals[idx])
+    op = geo.ThermalOperator(geo.Mesh(xyz, conn), dm, np.full(conn.shape[0], 3.0))
+    fb = op.lift_rhs(np.zeros(xyz.shape[0]))
+    x, st = op.solve(fb, geo.ConjugateGradient().with_tolerance(1e-12).with_max_iterations(limit).with_precision(precision))
+    assert st.iterations == limit and not st.converged
+    # the solution left behind belongs to the last iteration: its residual is the one reported
+    true = np.linalg.norm(fb - op.apply(x))
+    bar = 1e-9 if precision == "fp64" else 1e-5  # rounding of the recursion; of the FP32 correction
+    assert abs(true - st.residual_norm) <= bar * np.linalg.norm(fb)
