@@ -940,39 +940,6 @@ geo_op* create_op(geo_ctx* ctx, const geo_mesh* mesh, const geo_dofs* dofs, int 
     return op.release();
 }
 
-// y = K_bc x in patch numbering (device vectors of type T)
-template <class T>
-void apply_new(geo_op* op, const T* x, T* y, int mode) {
-    geo_ctx* ctx = op->ctx;
-    cudaStream_t s = ctx->stream;
-    GEO_CUDA(cudaMemsetAsync(y, 0, op->ndof * sizeof(T), s));
-    constexpr bool dbl = std::is_same<T, double>::value;
-    const bool halo = op->halo[dbl ? 0 : 1] != 0;
-    reset_dev_err(ctx);
-    with_kernels(op, [&](auto k64, auto k32) {
-        using K = typename std::conditional<dbl, decltype(k64), decltype(k32)>::type;
-        const T* qd = dbl ? (const T*)op->qd64.p : (const T*)op->qd32.p;
-        PatchArgs<T> pa{};
-        pa.x = x;
-        pa.y = y;
-        pa.err = ctx->dev_err.p;
-        if (halo) pa.halo = dbl ? (T*)op->halo64.p : (T*)op->halo32.p;
-        if (mode == MODE_FREE) launch_patch<K, T, MODE_FREE>(op, dbl ? 0 : 1, s, qd, pa);
-        else launch_patch<K, T, MODE_LIFT>(op, dbl ? 0 : 1, s, qd, pa);
-    });
-    check_launch(ctx, "k_patch");
-    if (halo) {  // foreign contributions in slot order (and the Dirichlet rows of FREE)
-        const T* h = dbl ? (const T*)op->halo64.p : (const T*)op->halo32.p;
-        k_halo_combine<T><<<nblk(op->N), kNodeBS, 0, s>>>(op->flags.p, op->hbase.p, h, op->dpn, op->N, op->cd, x,
-                                                          y, mode == MODE_FREE);
-        check_launch(ctx, "k_halo_combine");
-    } else if (mode == MODE_FREE) {
-        k_dir_rows<T><<<nblk(op->ndof), 256, 0, s>>>(op->flags.p, op->dpn, op->ndof, op->cd, x, y);
-        check_launch(ctx, "k_dir_rows");
-    }
-    raise_dev_err(ctx, read_dev_err(ctx), "matrix-free apply");
-}
-
 void to_new(geo_op* op, const double* in_orig, double* out_new) {
     k_to_new<double, double><<<nblk(op->ndof), 256, 0, op->ctx->stream>>>(op->nperm.p, op->dpn, op->N, in_orig,
                                                                           out_new);
@@ -984,17 +951,84 @@ void to_orig(geo_op* op, const double* in_new, double* out_orig) {
     check_launch(op->ctx, "k_to_orig");
 }
 
-// f_bc (patch numbering) from f (original numbering), device buffers
+// The patch pass y = K x (MODE_FREE) or K g (MODE_LIFT) in patch numbering, device vectors
+// of type T, foreign contributions in the halo slots in halo mode. A wait that runs out
+// shows in ctx->dev_err, which the caller reads with its results.
+template <class T>
+void patch_pass(geo_op* op, const T* x, T* y, int mode) {
+    geo_ctx* ctx = op->ctx;
+    cudaStream_t s = ctx->stream;
+    constexpr int slot = std::is_same<T, double>::value ? 0 : 1;
+    if (!op->halo[slot]) GEO_CUDA(cudaMemsetAsync(y, 0, op->ndof * sizeof(T), s));
+    reset_dev_err(ctx);
+    with_kernels(op, [&](auto k64, auto k32) {
+        using K = typename std::conditional<slot == 0, decltype(k64), decltype(k32)>::type;
+        const T* qd = slot == 0 ? (const T*)op->qd64.p : (const T*)op->qd32.p;
+        PatchArgs<T> pa{};
+        pa.x = x;
+        pa.y = y;
+        pa.err = ctx->dev_err.p;
+        if (op->halo[slot]) pa.halo = slot == 0 ? (T*)op->halo64.p : (T*)op->halo32.p;
+        if (mode == MODE_FREE) launch_patch<K, T, MODE_FREE>(op, slot, s, qd, pa);
+        else launch_patch<K, T, MODE_LIFT>(op, slot, s, qd, pa);
+    });
+    check_launch(ctx, "k_patch");
+}
+
+template <class T, class F>
+void halo_finish(geo_op* op, const T* y, const F& fin) {
+    const T* h = std::is_same<T, double>::value ? (const T*)op->halo64.p : (const T*)op->halo32.p;
+    k_halo_finish<T, F><<<nblk(op->N), kNodeBS, 0, op->ctx->stream>>>(op->flags.p, op->hbase.p, h, op->nperm.p, op->dpn,
+                                                                      op->N, y, fin);
+    check_launch(op->ctx, "k_halo_finish");
+}
+
+// y = K_bc x, both in the original numbering (device), x and y of the pass in patch
+// numbering in xn, yn.
+template <class T>
+void apply_orig(geo_op* op, const double* x, T* xn, T* yn, double* y) {
+    cudaStream_t s = op->ctx->stream;
+    const int64_t n = op->ndof;
+    k_to_new<double, T><<<nblk(n), 256, 0, s>>>(op->nperm.p, op->dpn, op->N, x, xn);
+    check_launch(op->ctx, "k_to_new");
+    patch_pass<T>(op, xn, yn, MODE_FREE);
+    if (op->halo[std::is_same<T, double>::value ? 0 : 1]) {
+        halo_finish(op, yn, ApplyOut<T>{op->cd, xn, y});
+    } else {
+        k_dir_rows<T><<<nblk(n), 256, 0, s>>>(op->flags.p, op->dpn, n, op->cd, xn, yn);
+        k_to_orig<T, double><<<nblk(n), 256, 0, s>>>(op->nperm.p, op->dpn, op->N, yn, y);
+        check_launch(op->ctx, "k_to_orig");
+    }
+}
+
+// f_bc (patch numbering) from f (original numbering), device buffers. The caller calls
+// check_pass when it has synchronised anyway.
 void lift_new(geo_op* op, const double* f_orig_dev, double* fbc_new) {
     cudaStream_t s = op->ctx->stream;
-    double* fn = grow(op->tmp[4], (size_t)op->ndof);
     double* kg = grow(op->tmp[5], (size_t)op->ndof);
-    to_new(op, f_orig_dev, fn);
-    apply_new<double>(op, op->g_new.p, kg, MODE_LIFT);
-    k_lift_finish<<<nblk(op->ndof), 256, 0, s>>>(op->flags.p, op->dpn, op->ndof, op->cd, fn, op->g_new.p, kg,
-                                                fbc_new);
-    check_launch(op->ctx, "k_lift_finish");
-    sync(op->ctx, "lift");
+    patch_pass<double>(op, op->g_new.p, kg, MODE_LIFT);
+    if (op->halo[0]) {
+        halo_finish(op, kg, LiftOut{op->cd, f_orig_dev, op->g_new.p, fbc_new});
+    } else {
+        double* fn = grow(op->tmp[4], (size_t)op->ndof);
+        to_new(op, f_orig_dev, fn);
+        k_lift_finish<<<nblk(op->ndof), 256, 0, s>>>(op->flags.p, op->dpn, op->ndof, op->cd, fn, op->g_new.p, kg,
+                                                    fbc_new);
+        check_launch(op->ctx, "k_lift_finish");
+    }
+}
+
+// Synchronises and raises what a patch_pass reported.
+void check_pass(geo_op* op, const char* what) { raise_dev_err(op->ctx, read_dev_err(op->ctx), what); }
+
+// p is memory of the context's device, which a kernel may write in place of a copy.
+bool on_device(const geo_op* op, const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == op->ctx->device;
 }
 
 // Blocks of a node kernel whose threads take `items` items: one wave of resident
@@ -1378,25 +1412,12 @@ int geo_op_apply(geo_op* op, const double* x, double* y, int32_t precision) {
     cudaStream_t s = op->ctx->stream;
     const int64_t n = op->ndof;
     const double* dx = stage_in(x, n, op->tmp[0], s);
-    double* yo = grow(op->tmp[3], (size_t)n);
-    if (precision == GEO_PRECISION_MIXED) {
-        float* x32 = grow(op->tmp32[0], (size_t)n);
-        float* y32 = grow(op->tmp32[1], (size_t)n);
-        k_to_new<double, float><<<nblk(n), 256, 0, s>>>(op->nperm.p, op->dpn, op->N, dx, x32);
-        apply_new<float>(op, x32, y32, MODE_FREE);
-        k_to_orig<float, double><<<nblk(n), 256, 0, s>>>(op->nperm.p, op->dpn, op->N, y32, yo);
-        check_launch(op->ctx, "k_to_orig");
-        copy_out(y, yo, n, s);
-        sync(op->ctx, "geo_op_apply");
-    } else {
-        double* xn = grow(op->tmp[1], (size_t)n);
-        double* yn = grow(op->tmp[2], (size_t)n);
-        to_new(op, dx, xn);
-        apply_new<double>(op, xn, yn, MODE_FREE);
-        to_orig(op, yn, yo);
-        copy_out(y, yo, n, s);
-        sync(op->ctx, "geo_op_apply");
-    }
+    double* yo = on_device(op, y) ? y : grow(op->tmp[3], (size_t)n);
+    if (precision == GEO_PRECISION_MIXED)
+        apply_orig<float>(op, dx, grow(op->tmp32[0], (size_t)n), grow(op->tmp32[1], (size_t)n), yo);
+    else apply_orig<double>(op, dx, grow(op->tmp[1], (size_t)n), grow(op->tmp[2], (size_t)n), yo);
+    if (yo != y) copy_out(y, yo, n, s);
+    check_pass(op, "matrix-free apply");
     GEO_API_END
 }
 
@@ -1407,11 +1428,11 @@ int geo_op_lift_rhs(geo_op* op, const double* f, double* f_bc) {
     const int64_t n = op->ndof;
     const double* df = stage_in(f, n, op->tmp[0], s);
     double* fb = grow(op->tmp[1], (size_t)n);
-    double* fo = grow(op->tmp[2], (size_t)n);
+    double* fo = on_device(op, f_bc) ? f_bc : grow(op->tmp[2], (size_t)n);
     lift_new(op, df, fb);
     to_orig(op, fb, fo);
-    copy_out(f_bc, fo, n, s);
-    sync(op->ctx, "geo_op_lift_rhs");
+    if (fo != f_bc) copy_out(f_bc, fo, n, s);
+    check_pass(op, "matrix-free lift");
     GEO_API_END
 }
 
@@ -1475,7 +1496,7 @@ int geo_forward(geo_op* op, const double* f, const geo_cg_opts* opts, double* u,
     if (!is_device_ptr(u)) dst = grow(op->tmp[1], (size_t)n);
     to_orig(op, op->xvec.p, dst);
     if (dst != u) copy_out(u, dst, n, s);
-    sync(op->ctx, "geo_forward");
+    check_pass(op, "matrix-free lift");
     return finish_status(op->ctx, status);
     GEO_API_END
 }
@@ -1498,6 +1519,7 @@ int geo_vjp(geo_op* op, const double* f, const double* u, const double* dJ_du, c
         const double* df = stage_in(f, n, op->tmp[0], s);
         lift_new(op, df, op->bvec.p);
         const int fs = solve_new(op, o, nullptr);
+        check_pass(op, "matrix-free lift");
         if (fs != GEO_OK) return finish_status(op->ctx, fs);
         double* uo = grow(op->tmp[2], (size_t)n);
         to_orig(op, op->xvec.p, uo);
