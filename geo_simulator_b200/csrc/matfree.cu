@@ -145,8 +145,7 @@ __global__ void k_qdata(int phys, const double* xyz, const int32_t* conn, const 
         }
         adj3(J, A);
         if (phys == 0) {
-            // affine elements: 4/5 of the rule's G (ThermalK::apply_affine)
-            const double s = (NQ == 1 ? 0.8 * kQw : kQw) * k / fabs(d);
+            const double s = kQw * k / fabs(d);
             double G[6];
             G[0] = s * (A[0][0] * A[0][0] + A[0][1] * A[0][1] + A[0][2] * A[0][2]);
             G[1] = s * (A[0][0] * A[1][0] + A[0][1] * A[1][1] + A[0][2] * A[1][2]);
@@ -156,7 +155,7 @@ __global__ void k_qdata(int phys, const double* xyz, const int32_t* conn, const 
             G[5] = s * (A[2][0] * A[2][0] + A[2][1] * A[2][1] + A[2][2] * A[2][2]);
             for (int j = 0; j < 6; ++j) {
                 const int64_t at = ((ne / kPatchElems) * (6 * NQ) + 6 * q + j) * kPatchElems + ne % kPatchElems;
-                qd64[at] = G[j];
+                qd64[at] = NQ == 1 ? 0.8 * G[j] : G[j];  // see ThermalK::apply_affine
                 qd32[at] = (float)G[j];
             }
         } else {

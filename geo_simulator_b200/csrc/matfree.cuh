@@ -11,8 +11,8 @@ namespace geo {
 // Per-element geometric data ("qdata"), stored patch-major: for patch p, value j
 // of the patch's element e sits at [(p * NQD + j) * kPatchElems + e]. Thermal: the
 // symmetric 3x3 G = (k w / |det J|) adj(J) adj(J)^T packed as [xx xy xz yy yz zz], per
-// quadrature point for curved elements (NQ = 4), once and times 4/5 for affine
-// elements (NQ = 1, see apply_affine). Elasticity: J^{-1} (9, row-major) and
+// quadrature point for curved elements (NQ = 4), once for affine elements (NQ = 1; in FP64
+// times 4/5, see apply_affine). Elasticity: J^{-1} (9, row-major) and
 // s = w |det J| E_e, once or per quadrature point.
 template <class T, int NQ>
 struct ThermalK {
@@ -20,16 +20,21 @@ struct ThermalK {
     static constexpr int NQD = 6 * NQ;
 
     // y = S K_e x. qd points at the element's first qdata value; value j sits at qd[j * stride].
+    // The FP32 PCG takes the affine form like FP64 (128^3: 248 us per launch against 254
+    // point by point): its rounding is the refinement's to correct. The FP32 operator apply
+    // hands its rounding to the caller and keeps the point by point form (NQ == 1: one G for
+    // the four points).
+    template <bool PCG = false>
     __device__ __forceinline__ static void apply(const T* __restrict__ qd, int64_t stride, T, T, T S,
                                                  const T (&x)[10], T (&y)[10]) {
-        if (NQ == 1) apply_affine(qd, stride, S, x, y);
+        if (NQ == 1 && (sizeof(T) == 8 || PCG)) apply_affine(qd, stride, sizeof(T) == 8 ? S : T(0.8) * S, x, y);
         else apply_quadrature(qd, stride, S, x, y);
     }
 
     // Affine element: the gradient is linear in L, so with its values c_m at the four
     // vertices, int grad.G.grad = sum_mn (1 + delta_mn) / 20 c_m.G c_n: the exact value
-    // of the 4-point rule. qdata holds 4/5 of the rule's G (4 points / 20 x 4, the factor
-    // 4 of the gradients folded in). 114 operations, against 132 for the point by point form.
+    // of the 4-point rule, on 4/5 of the rule's G (4 points / 20 x 4, the factor 4 of the
+    // gradients folded in), which the FP64 qdata holds and S brings to the FP32 one. 114 operations, against 132 for the point by point form.
     __device__ __forceinline__ static void apply_affine(const T* __restrict__ qd, int64_t stride, T S,
                                                         const T (&x)[10], T (&y)[10]) {
         T G[6];
@@ -86,7 +91,7 @@ struct ThermalK {
         for (int q = 0; q < 4; ++q) {
             T G[6];
 #pragma unroll
-            for (int j = 0; j < 6; ++j) G[j] = qd[(6 * q + j) * stride];
+            for (int j = 0; j < 6; ++j) G[j] = qd[(NQ == 1 ? j : 6 * q + j) * stride];
             T h[4];
 #pragma unroll
             for (int m = 0; m < 4; ++m) h[m] = base[m] + D4 * (m == q ? x[m] : x[edge_of(m, m == q ? (q + 1) % 4 : q)]);
@@ -118,6 +123,7 @@ struct ElasticK {
 
     // x, y interleaved [3*i + c]; cl = nu/((1+nu)(1-2nu)), cm = 1/(2(1+nu))
     // y = S K_e x; S is applied to y last: times the element's stiffness it could overflow
+    template <bool PCG = false>
     __device__ __forceinline__ static void apply(const T* __restrict__ qd, int64_t stride, T cl, T cm, T S,
                                                  const T (&x)[30], T (&y)[30]) {
         const T B4 = T(4.0 * kQb), D4 = T(4.0 * (kQa - kQb)), B4m1 = T(4.0 * kQb - 1.0);

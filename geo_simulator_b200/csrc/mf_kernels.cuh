@@ -885,11 +885,12 @@ __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
             }
             const float bx = __fmul_ru(pm.bound, __fmaf_ru(mabs, 1.52587890625e-05f, half));  // 2^-16
             if (bx > 0.0f) {
-                // S multiplies G of the affine thermal elements (ThermalK::apply_affine): it
-                // stays below 2^120 / bound, and G below the bound on K_e's norm
+                // S multiplies G of the affine thermal elements in the FP32 PCG
+                // (ThermalK::apply_affine): it stays below 2^120 / bound, and G below the
+                // bound on K_e's norm
                 const int cap = min(100, 246 - (int)(__float_as_uint(pm.bound) >> 23));
                 float sf, isf;
-                pow2_scale(bx, Scatter<T>::kLimExp, DPN == 1 && sizeof(T) == 4 ? cap : 100, sf, isf);
+                pow2_scale(bx, Scatter<T>::kLimExp, MODE == MODE_PCG && DPN == 1 && sizeof(T) == 4 ? cap : 100, sf, isf);
                 S = (T)sf;
                 invS = (T)isf;
             }
@@ -913,7 +914,7 @@ __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
             for (int l = 0; l < 10; ++l)
 #pragma unroll
                 for (int c = 0; c < DPN; ++c) xe[l * DPN + c] = tab.x(h[l], c);
-            K::apply(qds + el, kPatchElems, cl, cm, S, xe, ye);
+            K::template apply<MODE == MODE_PCG>(qds + el, kPatchElems, cl, cm, S, xe, ye);
             if (MODE == MODE_PCG) {
                 T d = T(0);
 #pragma unroll
