@@ -34,7 +34,8 @@ struct ThermalK {
     // Affine element: the gradient is linear in L, so with its values c_m at the four
     // vertices, int grad.G.grad = sum_mn (1 + delta_mn) / 20 c_m.G c_n: the exact value
     // of the 4-point rule, on 4/5 of the rule's G (4 points / 20 x 4, the factor 4 of the
-    // gradients folded in), which the FP64 qdata holds and S brings to the FP32 one. 114 operations, against 132 for the point by point form.
+    // gradients folded in), which the FP64 qdata holds and S brings to the FP32 one. 114
+    // operations, against 132 for the point by point form.
     __device__ __forceinline__ static void apply_affine(const T* __restrict__ qd, int64_t stride, T S,
                                                         const T (&x)[10], T (&y)[10]) {
         T G[6];
