@@ -1585,7 +1585,7 @@ __global__ void __launch_bounds__(kNodeBS) k_refresh_residual_halo(NodeArgs<floa
 // the original one (nperm: new node -> original). Every node is some patch's own, so the
 // pass has stored all of y. Node-per-thread with warp-aligned 32-node chunks (grid a
 // multiple of 32 threads). fin writes the caller's vector, which saves a pass over y and,
-// at 45x37x29 (0.41 M dofs, FP64), the launches and copies around it: operator apply 110 ->
+// at 45x37x29 (0.40 M dofs, FP64), the launches and copies around it: operator apply 108 ->
 // 85 us.
 template <class T, class F>
 __global__ void __launch_bounds__(kNodeBS) k_halo_finish(const uint8_t* __restrict__ flags,
