@@ -480,9 +480,10 @@ struct geo_op {
     int own_bulk[2] = {0, 0};          // own-node slices by bulk copy (PCG), see setup
     size_t patch_smem[2] = {0, 0};     // dynamic shared memory of the patch kernel
     int node_grid[2] = {0, 0};  // resident node-kernel blocks (FP64, mixed)
-    // CUDA graphs of the PCG loop, keyed by precision
+    // CUDA graphs of the PCG loop by precision, and the workspaces each one was built on: the
+    // buffers in it that can move while the operator lives (pcg_args grows them)
     cudaGraphExec_t loop[2] = {nullptr, nullptr};
-    const void* loop_key[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    const void* loop_on[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     ~geo_op() {
         for (auto& g : loop)
             if (g) cudaGraphExecDestroy(g);
@@ -1252,7 +1253,6 @@ cudaGraphExec_t build_loop(geo_op* op, bool mixed, const PcgLaunchArgs& la) {
 // that the device steers; the host reads the state when it has ended.
 int solve_new(geo_op* op, const geo_cg_opts& o, geo_solver_stats* st) {
     geo_ctx* ctx = op->ctx;
-    double* x_new = op->xvec.p;
     cudaStream_t s = ctx->stream;
     GEO_CHECK_ARG(o.use_preconditioner, "the matrix-free solver is Jacobi-preconditioned only");
     const bool mixed = o.precision == GEO_PRECISION_MIXED;
@@ -1268,16 +1268,16 @@ int solve_new(geo_op* op, const geo_cg_opts& o, geo_solver_stats* st) {
     const unsigned ng = node_blocks(op, mixed ? 1 : 0, op->ndof);
     GEO_CUDA(cudaEventRecord(ctx->ev0, s));
     pcg_start(op, mixed, init, la);
-    // (re)build the loop's graph when the buffers it captured changed
+    // (re)build the loop's graph when a buffer that it captured has moved: an FP64 solve, or
+    // the timing of one, grows w64, which the mixed loop's refresh works in
     const int pi = mixed ? 1 : 0;
-    const void* key0 = mixed ? (const void*)op->w32.p : (const void*)op->w64.p;
-    const void* key1 = (const void*)x_new;
-    if (!op->loop[pi] || op->loop_key[pi][0] != key0 || op->loop_key[pi][1] != key1) {
+    const void* on[2] = {op->w64.p, mixed ? op->w32.p : nullptr};
+    if (!op->loop[pi] || op->loop_on[pi][0] != on[0] || op->loop_on[pi][1] != on[1]) {
         if (op->loop[pi]) cudaGraphExecDestroy(op->loop[pi]);
         op->loop[pi] = nullptr;
         op->loop[pi] = build_loop(op, mixed, la);
-        op->loop_key[pi][0] = key0;
-        op->loop_key[pi][1] = key1;
+        op->loop_on[pi][0] = on[0];
+        op->loop_on[pi][1] = on[1];
     }
     GEO_CUDA(cudaGraphLaunch(op->loop[pi], s));
     GEO_CUDA(cudaMemcpyAsync(op->h_state, op->state.p, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
