@@ -78,7 +78,8 @@ __global__ void k_inc_sort(const int32_t* __restrict__ ptr, int32_t* __restrict_
 // One warp per node row: gather candidate columns, bitonic sort, count / emit
 // the distinct ones and, with out_pos, the places of every incident element's nodes
 // among them (geo_mesh::pat_pos). err[0] gets DEV_ERR_BOUNDS when a row exceeds
-// kPatCap, err[1] the largest row beyond 256.
+// kPatCap, err[1] the largest row beyond 256, err[2] is set when an element lists a node
+// twice (two neighbouring incidences of the node, which are sorted by element).
 __global__ void __launch_bounds__(32 * kPatWarps)
 k_pattern(const int32_t* __restrict__ conn, int64_t E, const int32_t* __restrict__ ptr,
           const int32_t* __restrict__ inc, int64_t N, int64_t* __restrict__ row_cnt,
@@ -143,6 +144,9 @@ k_pattern(const int32_t* __restrict__ conn, int64_t E, const int32_t* __restrict
             row_cnt[i] = run;
             if (run > 256) atomicMax(err + 1, run);
         }
+        if (row_cnt)
+            for (int t = lane; t + 1 < deg; t += 32)
+                if (inc[b + t] / 10 == inc[b + t + 1] / 10) atomicOr(err + 2, 1);
         if (out_pos)
             for (int t = lane; t < 3 * deg; t += 32) {  // word t % 3 of incidence t / 3
                 const int64_t e = inc[b + t / 3] / 10;
@@ -288,7 +292,23 @@ struct RowArgs {
     double* data;
     double lam, mu;
     int64_t lo, hi;  // the launch takes the blocks of more than lo and at most hi entries
+    bool repeats;    // some element lists a node twice: two of its columns are one entry
 };
+
+// row[at[j]] += y[j] for an element's ten columns: all loads, then all stores, where they
+// are distinct entries; one after the other where two may be the same.
+__device__ __forceinline__ void add_columns(double* row, const int (&at)[10], const double (&y)[10], bool repeats) {
+    if (repeats) {
+#pragma unroll
+        for (int j = 0; j < 10; ++j) row[at[j]] = __dadd_rn(row[at[j]], y[j]);
+        return;
+    }
+    double v[10];
+#pragma unroll
+    for (int j = 0; j < 10; ++j) v[j] = row[at[j]];
+#pragma unroll
+    for (int j = 0; j < 10; ++j) row[at[j]] = __dadd_rn(v[j], y[j]);
+}
 
 // Place of the element's local node j in its row: from the pattern's bytes, or by
 // search in the row [rb, re).
@@ -362,15 +382,10 @@ __global__ void __launch_bounds__(kRowsT) k_thermal_rows(RowArgs a) {
                     y[4 + k] += 4.0 * (n == q ? kQa : kQb) * f[m] + 4.0 * (m == q ? kQa : kQb) * f[n];
                 }
             }
-            // the element's columns are distinct: all loads, then all stores
             int at[10];
-            double v[10];
 #pragma unroll
             for (int j = 0; j < 10; ++j) at[j] = row_place<SMEM>(a, w, j, e, rb, re);
-#pragma unroll
-            for (int j = 0; j < 10; ++j) v[j] = row[at[j]];
-#pragma unroll
-            for (int j = 0; j < 10; ++j) row[at[j]] = __dadd_rn(v[j], y[j]);
+            add_columns(row, at, y, a.repeats);
         }
     }
     if (SMEM) {
@@ -462,17 +477,15 @@ __global__ void __launch_bounds__(3 * kRowsE) k_elastic_rows(RowArgs a) {
                     }
                 }
             }
-            // the element's columns are distinct: all loads of a component, then all stores
             int at[10];
 #pragma unroll
             for (int j = 0; j < 10; ++j) at[j] = 3 * row_place<SMEM>(a, w, j, e, rb, re);
 #pragma unroll
             for (int b = 0; b < 3; ++b) {
-                double v[10];
+                double y[10];
 #pragma unroll
-                for (int j = 0; j < 10; ++j) v[j] = row[at[j] + b];
-#pragma unroll
-                for (int j = 0; j < 10; ++j) row[at[j] + b] = __dadd_rn(v[j], K[j][b]);
+                for (int j = 0; j < 10; ++j) y[j] = K[j][b];
+                add_columns(row + b, at, y, a.repeats);
             }
         }
     }
@@ -512,7 +525,7 @@ void launch_rows(geo_ctx* ctx, const geo_mesh* m, int per_entry, int64_t block_m
     const int threads = per_entry == 1 ? ROWS : 3 * ROWS;
     const unsigned g = blocks(m->n_nodes, ROWS);
     RowArgs a{m->conn.p, m->inc_ptr.p, m->inc.p, m->pat_ptr.p, m->pat_idx.p, m->pat_pos.p, metric,
-              m->n_nodes, m->n_elem, indices, data, lam, mu, 0, 0};
+              m->n_nodes, m->n_elem, indices, data, lam, mu, 0, 0, m->pat_repeats};
     int64_t done = -1;  // blocks of at most this many entries are launched
     if (m->pat_pos.p) {
         GEO_CUDA(cudaFuncSetAttribute(smem_form, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMost * 8)));
@@ -676,12 +689,12 @@ void ensure_pattern(geo_mesh* m) {
     const int64_t N = m->n_nodes, E = m->n_elem;
     DevBuf<int64_t> cnt(N + 1);
     GEO_CUDA(cudaMemsetAsync(cnt.p, 0, (N + 1) * sizeof(int64_t), s));
-    GEO_CUDA(cudaMemsetAsync(ctx->dev_err.p, 0, 2 * sizeof(int), s));
+    GEO_CUDA(cudaMemsetAsync(ctx->dev_err.p, 0, 3 * sizeof(int), s));
     const unsigned g = (unsigned)std::min<int64_t>(cdiv(N, kPatWarps), 1 << 20);
     k_pattern<<<g, 32 * kPatWarps, 0, s>>>(m->conn.p, E, m->inc_ptr.p, m->inc.p, N, cnt.p, nullptr, nullptr, nullptr,
                                            ctx->dev_err.p);
     check_launch(ctx, "k_pattern(count)");
-    int h[2] = {0, 0};  // error bits, largest row
+    int h[3] = {0, 0, 0};  // error bits, largest row, repeated nodes
     GEO_CUDA(cudaMemcpyAsync(h, ctx->dev_err.p, sizeof h, cudaMemcpyDeviceToHost, s));
     sync(ctx, "pattern counts");
     if (h[0] & DEV_ERR_BOUNDS)
@@ -699,6 +712,7 @@ void ensure_pattern(geo_mesh* m) {
     sync(ctx, "pattern size");
     m->pat_block_t = (int64_t)hb[0];
     m->pat_block_e = (int64_t)hb[1];
+    m->pat_repeats = h[2] != 0;
     m->pat_idx.alloc(nnz);
     if (h[1] <= 256) m->pat_pos.alloc(30 * (size_t)E);
     k_pattern<<<g, 32 * kPatWarps, 0, s>>>(m->conn.p, E, m->inc_ptr.p, m->inc.p, N, nullptr, m->pat_ptr.p,

@@ -75,6 +75,7 @@ struct geo_mesh {
     geo::DevBuf<uint32_t> pat_pos;
     // most entries of any block of consecutive rows: thermal and elastic value kernels
     int64_t pat_block_t = 0, pat_block_e = 0;
+    bool pat_repeats = false;  // some element lists a node twice
 };
 
 struct geo_dofs {
