@@ -77,11 +77,19 @@ struct LuArgs {
     int32_t* piv;          // piv[k]: the row eliminated at column k
     double* lbuf;          // [m][nb] multipliers, in list_out's order
     double* l11;           // [kMaxNb][kMaxNb] the panel's unit lower triangle
-    int* singular;
+    int* singular;         // 0, or 1 + the first column of the panel that met a zero pivot
     double* x;             // the solution
     GridSync* gs;
     unsigned long long timeout_ns;
 };
+
+// This panel, or one before it, met a zero pivot. The panel after it may find one while the
+// rest of this one's trailing update runs beside it (see lu_panel), which must not stop some
+// threads of a block and not others.
+__device__ __forceinline__ bool panel_failed(const LuArgs& a) {
+    const int at = cuda::atomic_ref<int, cuda::thread_scope_device>(*a.singular).load(cuda::memory_order_relaxed);
+    return at != 0 && at <= a.k0 + 1;
+}
 
 // Bits of +infinity: |v| as an integer is above it for NaN, and at least it for both.
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
@@ -134,7 +142,7 @@ __global__ void __launch_bounds__(kPanelBS) k_lu_panel(LuArgs a) {
     __shared__ double s_row[kMaxNb];
     __shared__ double s_up[NB][NB];  // block 0: the pivot rows from their column on
     __shared__ int s_piv[NB];
-    if (*a.singular) return;  // set by an earlier panel: the same for every block
+    if (panel_failed(a)) return;  // an earlier panel: the same for every block
     cg::cluster_group cluster = cg::this_cluster();
     const int ncta = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     const int bs = blockDim.x, nwarp = bs >> 5;
@@ -296,7 +304,8 @@ __global__ void __launch_bounds__(kPanelBS) k_lu_panel(LuArgs a) {
         careful = true;
         singular = false;
     }
-    if (singular && rank == 0 && threadIdx.x == 0) *a.singular = 1;
+    if (singular && rank == 0 && threadIdx.x == 0)
+        cuda::atomic_ref<int, cuda::thread_scope_device>(*a.singular).store(a.k0 + 1, cuda::memory_order_relaxed);
     __syncthreads();
     if (!singular) {
         if (rank == 0)
@@ -328,7 +337,7 @@ __global__ void __launch_bounds__(64) k_lu_rows(LuArgs a) {
     __shared__ double l[NB][NB];
     const int lane = threadIdx.x & 31;
     const int mine = lane < a.nbw ? a.piv[a.k0 + lane] : 0;  // pivot row `lane`
-    if (*a.singular) return;
+    if (panel_failed(a)) return;
     const int64_t j = a.k0 + a.nbw + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     double u[NB];
 #pragma unroll
@@ -377,7 +386,7 @@ __global__ void __launch_bounds__(128) k_lu_trailing(LuArgs a) {
     __shared__ double U[NB][kTile];
     __shared__ int s_wild;  // the tile's multipliers or pivot rows hold an infinity or a NaN
     if (threadIdx.x == 0) s_wild = 0;
-    if (*a.singular) return;
+    if (panel_failed(a)) return;
     const int m = a.m - a.nbw;  // rows left
     const int r0 = blockIdx.y * kTile;
     const int64_t c0 = a.k0 + a.nbw + (a.tile0 + (int64_t)blockIdx.x) * kTile;
