@@ -1021,8 +1021,10 @@ void lift_new(geo_op* op, const double* f_orig_dev, double* fbc_new) {
 // Synchronises and raises what a patch_pass reported.
 void check_pass(geo_op* op, const char* what) { raise_dev_err(op->ctx, read_dev_err(op->ctx), what); }
 
-// p is memory of the context's device, which a kernel may write in place of a copy.
-bool on_device(const geo_op* op, const void* p) {
+// p is memory of the context's device, which a kernel may write in place of a copy: aligned
+// for doubles too, which a copy does not ask for.
+bool on_device(const geo_op* op, const double* p) {
+    if (reinterpret_cast<uintptr_t>(p) % alignof(double) != 0) return false;
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
