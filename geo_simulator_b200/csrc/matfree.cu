@@ -579,7 +579,8 @@ void with_patch_kernel(int nbuf, int halo, F&& f) {
 
 // Lets a kernel take `bytes` of dynamic shared memory. The attribute belongs to the
 // kernel, not to the operator, so it is only ever raised: a smaller operator made later
-// must not take it from a larger one that is still in use.
+// must not take it from a larger one that is still in use. It is set each time, since a
+// cudaDeviceReset puts it back to its default.
 template <class Kernel>
 void allow_smem(Kernel k, size_t bytes) {
     static std::mutex mu;
@@ -588,9 +589,8 @@ void allow_smem(Kernel k, size_t bytes) {
     GEO_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(mu);
     size_t& a = allowed[{dev, (const void*)k}];
-    if (bytes <= a) return;
-    GEO_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    a = bytes;
+    a = std::max(a, bytes);
+    GEO_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a));
 }
 
 // Resident blocks per SM of the PCG-mode patch kernel.
