@@ -292,22 +292,23 @@ struct RowArgs {
     double* data;
     double lam, mu;
     int64_t lo, hi;  // the launch takes the blocks of more than lo and at most hi entries
-    bool repeats;    // some element lists a node twice: two of its columns are one entry
 };
 
 // row[at[j]] += y[j] for an element's ten columns: all loads, then all stores, where they
-// are distinct entries; one after the other where two may be the same.
-__device__ __forceinline__ void add_columns(double* row, const int (&at)[10], const double (&y)[10], bool repeats) {
-    if (repeats) {
+// are distinct entries; one after the other where two may be the same (REPEATS: some element
+// of the mesh lists a node twice).
+template <bool REPEATS>
+__device__ __forceinline__ void add_columns(double* row, const int (&at)[10], const double (&y)[10]) {
+    if constexpr (REPEATS) {
 #pragma unroll
         for (int j = 0; j < 10; ++j) row[at[j]] = __dadd_rn(row[at[j]], y[j]);
-        return;
+    } else {
+        double v[10];
+#pragma unroll
+        for (int j = 0; j < 10; ++j) v[j] = row[at[j]];
+#pragma unroll
+        for (int j = 0; j < 10; ++j) row[at[j]] = __dadd_rn(v[j], y[j]);
     }
-    double v[10];
-#pragma unroll
-    for (int j = 0; j < 10; ++j) v[j] = row[at[j]];
-#pragma unroll
-    for (int j = 0; j < 10; ++j) row[at[j]] = __dadd_rn(v[j], y[j]);
 }
 
 // Place of the element's local node j in its row: from the pattern's bytes, or by
@@ -326,9 +327,9 @@ __device__ __forceinline__ int row_place(const RowArgs& a, const uint32_t (&w)[3
 // updated it in global memory, and the 1.26 GB of element matrices (2.5 ms) give way to
 // 0.30 GB of geometry (0.17 ms). Bound by the L1 pipe: 192 bytes of geometry per
 // incidence and the conflicts of the accumulation.
-// SMEM = false (rows of more than 256 entries, or a block beyond shared memory) searches
-// and adds in global memory.
-template <bool SMEM>
+// SMEM = false (rows of more than 256 entries, a block beyond shared memory, REPEATS)
+// searches and adds in global memory.
+template <bool SMEM, bool REPEATS>
 __global__ void __launch_bounds__(kRowsT) k_thermal_rows(RowArgs a) {
     extern __shared__ double acc[];
     __shared__ double tab[120];
@@ -385,7 +386,7 @@ __global__ void __launch_bounds__(kRowsT) k_thermal_rows(RowArgs a) {
             int at[10];
 #pragma unroll
             for (int j = 0; j < 10; ++j) at[j] = row_place<SMEM>(a, w, j, e, rb, re);
-            add_columns(row, at, y, a.repeats);
+            add_columns<REPEATS>(row, at, y);
         }
     }
     if (SMEM) {
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(kRowsT) k_thermal_rows(RowArgs a) {
 // matrices, a searching row kernel and an index kernel. A warp per node with a lane per (c, j)
 // took 0.41 ms at 24x24x12: its sixteen indexed loads of gradients per element weigh more
 // than the divergence it avoids.
-template <bool SMEM>
+template <bool SMEM, bool REPEATS>
 __global__ void __launch_bounds__(3 * kRowsE) k_elastic_rows(RowArgs a) {
     extern __shared__ double acc[];
     __shared__ double tab[120];
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(3 * kRowsE) k_elastic_rows(RowArgs a) {
                 double y[10];
 #pragma unroll
                 for (int j = 0; j < 10; ++j) y[j] = K[j][b];
-                add_columns(row + b, at, y, a.repeats);
+                add_columns<REPEATS>(row + b, at, y);
             }
         }
     }
@@ -516,16 +517,17 @@ __global__ void k_elastic_indptr(const int64_t* __restrict__ pptr, int64_t N, in
 // few entries with little shared memory each, so that more of them are resident (the
 // vertices' rows of a Tet10 mesh are three times as long as the midpoints', in blocks of
 // their own), a second one the others; blocks beyond shared memory, and meshes without
-// the pattern's places, go through the global form.
+// the pattern's places, go through the global form, meshes with repeated nodes through their
+// own global form (a branch in the shared-memory form took it from 0.92 to 1.00 ms at 64^3).
 template <int ROWS, class K>
 void launch_rows(geo_ctx* ctx, const geo_mesh* m, int per_entry, int64_t block_max, K smem_form, K global_form,
-                 const double* metric, int32_t* indices, double* data, double lam, double mu) {
+                 K repeats_form, const double* metric, int32_t* indices, double* data, double lam, double mu) {
     cudaStream_t s = ctx->stream;
     const int64_t kMost = 200 * 1024 / 8;
     const int threads = per_entry == 1 ? ROWS : 3 * ROWS;
     const unsigned g = blocks(m->n_nodes, ROWS);
     RowArgs a{m->conn.p, m->inc_ptr.p, m->inc.p, m->pat_ptr.p, m->pat_idx.p, m->pat_pos.p, metric,
-              m->n_nodes, m->n_elem, indices, data, lam, mu, 0, 0, m->pat_repeats};
+              m->n_nodes, m->n_elem, indices, data, lam, mu, 0, 0};
     int64_t done = -1;  // blocks of at most this many entries are launched
     if (m->pat_pos.p) {
         GEO_CUDA(cudaFuncSetAttribute(smem_form, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMost * 8)));
@@ -542,7 +544,7 @@ void launch_rows(geo_ctx* ctx, const geo_mesh* m, int per_entry, int64_t block_m
     if (done < block_max) {
         a.lo = done;
         a.hi = INT64_MAX;
-        global_form<<<g, threads, 0, s>>>(a);
+        (m->pat_repeats ? repeats_form : global_form)<<<g, threads, 0, s>>>(a);
         check_launch(ctx, "row values (global)");
     }
 }
@@ -714,7 +716,7 @@ void ensure_pattern(geo_mesh* m) {
     m->pat_block_e = (int64_t)hb[1];
     m->pat_repeats = h[2] != 0;
     m->pat_idx.alloc(nnz);
-    if (h[1] <= 256) m->pat_pos.alloc(30 * (size_t)E);
+    if (h[1] <= 256 && !m->pat_repeats) m->pat_pos.alloc(30 * (size_t)E);
     k_pattern<<<g, 32 * kPatWarps, 0, s>>>(m->conn.p, E, m->inc_ptr.p, m->inc.p, N, nullptr, m->pat_ptr.p,
                                            m->pat_idx.p, m->pat_pos.p, ctx->dev_err.p);
     check_launch(ctx, "k_pattern(fill)");
@@ -774,8 +776,8 @@ int geo_assemble_thermal_stiffness(geo_ctx* ctx, const geo_mesh* mesh, const geo
     auto A = new_csr(ctx, N, N, m->pat_nnz);
     GEO_CUDA(cudaMemcpyAsync(A->indptr.p, m->pat_ptr.p, (N + 1) * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
     GEO_CUDA(cudaMemcpyAsync(A->indices.p, m->pat_idx.p, m->pat_nnz * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-    launch_rows<kRowsT>(ctx, m, 1, m->pat_block_t, k_thermal_rows<true>, k_thermal_rows<false>, G.p, A->indices.p,
-                        A->data.p, 0.0, 0.0);
+    launch_rows<kRowsT>(ctx, m, 1, m->pat_block_t, k_thermal_rows<true, false>, k_thermal_rows<false, false>,
+                        k_thermal_rows<false, true>, G.p, A->indices.p, A->data.p, 0.0, 0.0);
     raise_dev_err(ctx, read_dev_err(ctx), "thermal stiffness");
     *K = A.release();
     GEO_API_END
@@ -820,8 +822,8 @@ int geo_assemble_elasticity_stiffness(geo_ctx* ctx, const geo_mesh* mesh, const 
     check_launch(ctx, "k_elastic_indptr");
     // constitutive.rs:63-102 with the modulus in the metric
     const double lam = nu / ((1.0 + nu) * (1.0 - 2.0 * nu)), mu = 1.0 / (2.0 * (1.0 + nu));
-    launch_rows<kRowsE>(ctx, m, 9, 9 * m->pat_block_e, k_elastic_rows<true>, k_elastic_rows<false>, geom.p,
-                        A->indices.p, A->data.p, lam, mu);
+    launch_rows<kRowsE>(ctx, m, 9, 9 * m->pat_block_e, k_elastic_rows<true, false>,
+                        k_elastic_rows<false, false>, k_elastic_rows<false, true>, geom.p, A->indices.p, A->data.p, lam, mu);
     raise_dev_err(ctx, read_dev_err(ctx), "elasticity stiffness");
     *K = A.release();
     GEO_API_END

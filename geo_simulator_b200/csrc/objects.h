@@ -71,7 +71,7 @@ struct geo_mesh {
     int64_t pat_nnz = -1;
     // with the pattern: for every incidence p of inc the places of the element's 10 nodes
     // in the row of its node, one byte each in the words pat_pos[3 p .. 3 p + 2]; empty
-    // when some row has more than 256 entries
+    // when some row has more than 256 entries or some element lists a node twice
     geo::DevBuf<uint32_t> pat_pos;
     // most entries of any block of consecutive rows: thermal and elastic value kernels
     int64_t pat_block_t = 0, pat_block_e = 0;

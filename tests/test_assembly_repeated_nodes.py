@@ -1,7 +1,7 @@
 """CSR assembly of meshes with elements that list a node twice (an edge collapsed onto its
 end, two midpoints in one): both contributions reach the entry that the two columns share,
-in the row kernels' form with places in shared memory and in the searching form. Structure
-bit for bit, values against the oracle's triplet merge at 1e-12 of the row scale."""
+with and without a row of more than 256 entries. Structure bit for bit, values against the
+oracle's triplet merge at 1e-12 of the row scale."""
 import numpy as np
 import pytest
 
