@@ -516,7 +516,10 @@ __global__ void k_elastic_indptr(const int64_t* __restrict__ pptr, int64_t N, in
 // Launches a value kernel over all blocks of ROWS rows: a first launch takes the blocks of
 // few entries with little shared memory each, so that more of them are resident (the
 // vertices' rows of a Tet10 mesh are three times as long as the midpoints', in blocks of
-// their own), a second one the others; blocks beyond shared memory, and meshes without
+// their own), a second one the others. The line lies at 28 entries per row, the mean of a
+// Tet10 mesh, between the two kinds of block: one launch, 20, 28, 40, 60 entries take 1.01,
+// 1.03, 0.92, 0.98, 1.01 ms (thermal 64^3) and 0.37, 0.39, 0.26, 0.30, 0.42 ms (elastic
+// 24x24x12). Blocks beyond shared memory, and meshes without
 // the pattern's places, go through the global form, meshes with repeated nodes through their
 // own global form (a branch in the shared-memory form took it from 0.92 to 1.00 ms at 64^3).
 template <int ROWS, class K>

@@ -18,8 +18,9 @@
 //      subtracting its nb products in column order, as the unblocked elimination does:
 //      the blocked form changes no rounding. Tiles whose multipliers or pivot rows are
 //      all zero (a banded matrix) are skipped.
-// n = 3757 takes 12.1 ms (129 ms before, dense random matrices), n = 1000 2.7 ms (15.9): the unblocked form had two grid barriers and a pass over the trailing matrix per
-// column. Bound by the panels' chain of columns, about 1.9 us each.
+// n = 3757 takes 11.8 ms (127 ms before, dense random matrices), n = 1000 2.6 ms (15.6): the
+// unblocked form had two grid barriers and a pass over the trailing matrix per column.
+// Bound by the panels' chain of columns, about 1.9 us each.
 // Carrying b along leaves y = L^-1 P b in its column. Back substitution U x = y then
 // runs over 32-row blocks from the bottom in one persistent cooperative kernel: every
 // block solves the 32 x 32 diagonal triangle itself (one warp, identical in all blocks, so
@@ -545,7 +546,10 @@ template <int NB>
 int lu_panel(geo_ctx* ctx, LuArgs a, LookAhead* ahead) {
     cudaStream_t s = ahead ? ahead->s : ctx->stream;
     a.nbw = (int)std::min<int64_t>(NB, a.n - a.k0);
-    // blocks of at least two warps, spread over the cluster's SMs before they grow
+    // Blocks of at least two warps, spread over the cluster's SMs before they grow. A block
+    // for every 32, 64, 128, 256, 512 rows: n = 500 takes 1.22, 1.21, 1.20, 1.24, 1.33 ms,
+    // n = 2000 5.43, 5.41, 5.38, 5.44, 5.93: fewer, fuller blocks pay more for their own
+    // reductions than they save at the cluster barrier.
     constexpr int R = kPanelRegs / NB;
     int ncta = 1;
     while (ncta < kMaxCluster && ncta * 64 * R < a.m) ncta *= 2;
@@ -571,6 +575,7 @@ int lu_panel(geo_ctx* ctx, LuArgs a, LookAhead* ahead) {
     check_launch(ctx, "k_lu_rows");
     if (a.m == a.nbw) return 2;
     const unsigned ty = (unsigned)cdiv(a.m - a.nbw, kTile), tx = (unsigned)cdiv(cols, kTile);
+    // 2, 8 or 16 tile columns: within 0.3% of each other at n = 700 to 5000
     const bool split = ahead && tx > 8;
     if (split) GEO_CUDA(cudaEventRecord(ahead->rows, s));
     k_lu_trailing<NB><<<dim3(split ? 1 : tx, ty), 128, 0, s>>>(a);
@@ -631,6 +636,9 @@ int geo_direct_solve(geo_ctx* ctx, const geo_csr* A, const double* b, double* x,
     // rows at 32 columns, 8192 at 16, 16384 at 8).
     int64_t launches = 2;
     LookAhead ahead;
+    // Look-ahead costs a stream, two events and a split launch per panel: with and without,
+    // n = 300 0.77, 0.71 ms, 700 1.78, 1.72, 900 2.30, 2.25, 1200 3.08, 3.03, 1500 3.90, 3.90,
+    // 2000 5.42, 5.56, 3757 11.8, 14.2. It is even at 1500; the line at 640 is early by 3%.
     LookAhead* pa = n > 10 * kTile ? &ahead : nullptr;
     if (pa) {
         ahead.create();

@@ -496,8 +496,9 @@ namespace {
 
 // PCG iterations per pass of the graph's loop. A pass ends with k_pcg_decide and the loop's
 // own test (3 us together); the iterations behind a refresh or the end are launched as
-// no-ops. 4, 8, 16 per pass: 16^3 mixed 13.7, 12.9, 13.5 us per iteration, 48x48x32 mixed
-// 23.7, 23.0, 22.6, 64^3 FP64 93.8, 92.7, 92.2, elastic 48x48x24 mixed 41.7, 40.8, 40.4.
+// no-ops (see ST_IDLE). 8, 16 per pass: 6^3 FP64 solve 935, 900 us, 64^3 FP64 54.6, 54.2 ms,
+// viscoelastic step 27x22x13 13.1, 12.8, elastic 48x48x24 mixed 42.9, 42.5, inversion step
+// 48x48x32 35.6, 35.5; 4 per pass is slower still (16^3 FP64 by 6%).
 constexpr int kChunk = 16;
 
 inline unsigned nblk(int64_t n, int bs = 256) {
@@ -650,11 +651,16 @@ int setup_patch_kernels(geo_op* op, int slot) {
 
 // The PCG loop's kernels use programmatic dependent launch up to this many dofs: the next
 // kernel's blocks then start on the SMs that the last blocks of the one before leave, and
-// set up shared memory and the first patch's element copies before they wait. Per
-// iteration, without and with: 6^3 FP64 12.5 -> 11.6 us, 16^3 mixed 16.8 -> 15.1,
-// 48x48x32 mixed 24.1 -> 23.5, 64^3 FP64 (2.1 M dofs) 95.1 -> 92.6, elastic 48x48x24 mixed
-// (1.4 M) 41.5 -> 40.8. With more there is nothing to gain (elastic 48^3, 2.7 M: 169.8,
-// 169.7), and the mixed solver loses (thermal 80^3, 4.2 M: 96.7 -> 98.4; 128^3: 330 -> 342).
+// set up shared memory and the first patch's element copies before they wait. us per
+// iteration without and with, and M dofs:
+//   thermal FP64   40^3 (0.5) 32.3, 31.6; 56^3 (1.4) 73.2, 72.4; 64^3 (2.1) 93.9, 92.0;
+//                  72^3 (3.0) 148.3, 151.2; 88^3 (5.5) 253.8, 259.2
+//   thermal mixed  40^3 23.4, 22.0; 64^3 54.3, 52.8; 72^3 80.2, 79.3; 88^3 132.4, 130.2;
+//                  128^3 (17.0) 330, 342
+//   elastic FP64   32^3 (0.8) 59.0, 58.4; 44^3 (2.1) 137.7, 143.0; 52^3 (3.5) 224.6, 235.8
+//   elastic mixed  32^3 29.0, 27.9; 44^3 61.7, 61.4; 52^3 92.2, 92.4
+// One threshold for all four: it is right for thermal FP64 and elastic mixed; FP64
+// elasticity would end near 1 M, thermal mixed above 5.5 M.
 constexpr int64_t kDependentDofs = 2500000;
 
 // Launches k, with programmatic dependent launch when `dependent`: its blocks may start, up
@@ -737,7 +743,7 @@ void build_halo_slots(geo_op* op, int64_t seg_total) {
     if (total != A) fail(GEO_ERR_CUDA, "halo slot count mismatch");
     op->halo64.alloc(A * op->dpn);
     op->halo32.alloc(A * op->dpn);
-    // slots of Dirichlet entries are never written (the node update ignores them)
+    // every pass writes all slots, those of Dirichlet entries too (the node update ignores them)
     GEO_CUDA(cudaMemsetAsync(op->halo64.p, 0, op->halo64.bytes(), s));
     GEO_CUDA(cudaMemsetAsync(op->halo32.p, 0, op->halo32.bytes(), s));
     op->halo_ok = true;
@@ -1034,8 +1040,9 @@ bool on_device(const geo_op* op, const double* p) {
 }
 
 // Blocks of a node kernel whose threads take `items` items: one wave of resident
-// blocks, or as many as there is work for. Every block costs a ticket and a partial in
-// the last block's sum.
+// blocks, or as many as there is work for. Every block of the node update costs a partial
+// that all blocks of the next patch kernel add up (pcg_fold); one of the start and refresh
+// kernels a ticket and a partial in the last block's sum.
 unsigned node_blocks(const geo_op* op, int slot, int64_t items) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>(op->node_grid[slot], cdiv(items, kNodeBS)));
 }

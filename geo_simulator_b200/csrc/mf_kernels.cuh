@@ -88,7 +88,7 @@ struct PatchView {
     const uint8_t* fflags;
     int max_for;
     int max_own;   // the largest own-node count of a patch
-    int own_bulk;  // own-node slices by bulk copy (FP32 thermal PCG; the launch's shared memory holds them)
+    int own_bulk;  // PCG: own-node slices by bulk copy (the launch's shared memory holds them)
     // halo mode: the halo slot of every foreign entry, in the same per-patch segments as fids
     const int32_t* fslot;
     // per patch: element count, own range, foreign count and segment start, scatter
@@ -520,10 +520,11 @@ __host__ __device__ constexpr int patch_min_blocks() {
 // the foreign values requested before the flush of the patch before, one copy schedule
 // (late) for all kernels and the shorter affine apply, launches went from 264 to 249 us
 // (FP32 thermal, 128^3), 83 to 75 us (FP64 thermal, 64^3) and 37.3 to 33.2 us (FP32
-// elasticity, 48x48x24), events around each launch. The FP32 thermal kernel is bound by
-// the shared-memory pipe (67% of its wavefronts' peak, 4.4 per scatter atomic) and, at
-// 128^3, by the card's 1 kW power cap (clocks at 1.91 GHz); FP64 by latency (two blocks
-// of six warps per SM, issue 40%).
+// elasticity, 48x48x24), events around each launch. No unit is saturated: in the FP32
+// thermal kernel (96^3) the L1 data pipe, which gather and scatter share, is at 67% of its
+// peak (21 M wavefronts, 11 M of them bank conflicts, for 5.3 M elements), issue at 60%; at
+// 128^3 the card's 1 kW power cap holds the clock at 1.9 GHz. FP64: pipe 70%, issue 42%,
+// two blocks of six warps per SM.
 template <class K, class T, int MODE, int NBUF, int HM>
 __global__ void __launch_bounds__(kPatchBS, patch_min_blocks<K, T>())
     k_patch(PatchView pv, const T* __restrict__ qd_all, T cl, T cm, PatchArgs<T> a) {
