@@ -133,7 +133,7 @@ int geo_ctx_create(int device, geo_ctx** out) {
     GEO_CUDA(cudaEventCreate(&ctx->ev0));
     GEO_CUDA(cudaEventCreate(&ctx->ev1));
     ctx->dev_err.alloc(4);
-    GEO_CUDA(cudaMemset(ctx->dev_err.p, 0, 4 * sizeof(int)));
+    GEO_CUDA(cudaMemsetAsync(ctx->dev_err.p, 0, 4 * sizeof(int), ctx->stream));
     *out = ctx.release();
     GEO_API_END
 }

@@ -908,11 +908,15 @@ int geo_csr_create(geo_ctx* ctx, int64_t n_rows, int64_t n_cols, int64_t nnz, co
         }
     }
     auto A = new_csr(ctx, n_rows, n_cols, nnz);
-    GEO_CUDA(cudaMemcpy(A->indptr.p, hp.data(), (n_rows + 1) * sizeof(int64_t), cudaMemcpyHostToDevice));
+    GEO_CUDA(cudaMemcpyAsync(A->indptr.p, hp.data(), (n_rows + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
     if (nnz) {
-        GEO_CUDA(cudaMemcpy(A->indices.p, hi.data(), nnz * sizeof(int32_t), cudaMemcpyHostToDevice));
-        GEO_CUDA(cudaMemcpy(A->data.p, data, nnz * sizeof(double), cudaMemcpyDefault));
+        GEO_CUDA(cudaMemcpyAsync(A->indices.p, hi.data(), nnz * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
+        // behind the caller's work on the default stream, as the copies above that read it; the
+        // context's stream does not wait for that one by itself
+        GEO_CUDA(cudaMemcpyAsync(A->data.p, data, nnz * sizeof(double), cudaMemcpyDefault, cudaStreamLegacy));
+        GEO_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     }
+    sync(ctx, "geo_csr_create");
     *out = A.release();
     GEO_API_END
 }

@@ -885,7 +885,7 @@ geo_op* create_op(geo_ctx* ctx, const geo_mesh* mesh, const geo_dofs* dofs, int 
         if (acc > INT32_MAX) fail(GEO_ERR_UNSUPPORTED, "too many foreign patch nodes");
         pfa[P] = (int32_t)acc;
         op->pfa.alloc(P + 1);
-        GEO_CUDA(cudaMemcpy(op->pfa.p, pfa.data(), (P + 1) * sizeof(int32_t), cudaMemcpyHostToDevice));
+        GEO_CUDA(cudaMemcpyAsync(op->pfa.p, pfa.data(), (P + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, s));
         op->fids.alloc(acc + kForeignAlign);
         op->fflags.alloc(acc + kForeignAlign);
         GEO_CUDA(cudaMemsetAsync(op->fids.p, 0, op->fids.bytes(), s));
@@ -941,7 +941,7 @@ geo_op* create_op(geo_ctx* ctx, const geo_mesh* mesh, const geo_dofs* dofs, int 
     op->state.alloc(2);
     op->part.alloc((size_t)2 * std::max(op->node_grid[0], op->node_grid[1]));
     op->part_patch.alloc((size_t)2 * std::max(op->patch_grid[0], op->patch_grid[1]));
-    GEO_CUDA(cudaMemset(op->state.p, 0, op->state.bytes()));
+    GEO_CUDA(cudaMemsetAsync(op->state.p, 0, op->state.bytes(), s));
     GEO_CUDA(cudaMallocHost(&op->h_state, sizeof(PcgState)));
     return op.release();
 }
