@@ -18,6 +18,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <type_traits>
 #include <utility>
 
@@ -663,35 +664,68 @@ int setup_patch_kernels(geo_op* op, int slot) {
 // elasticity would end near 1 M, thermal mixed above 5.5 M.
 constexpr int64_t kDependentDofs = 2500000;
 
-// Launches k, with programmatic dependent launch when `dependent`: its blocks may start, up
-// to their griddepcontrol.wait, while the kernel before it in the stream still runs. Only
-// for kernels of the loop's graph: k_patch reads the operator's element data before its
-// wait, which must not be the output of the kernel before it.
+// A graph under construction whose nodes run one after the other. Built node by node, not
+// captured from a stream: a capture is lost when another thread of the process
+// synchronises the device meanwhile.
+struct GraphChain {
+    cudaGraph_t g;
+    cudaGraphNode_t last = nullptr;
+};
+
+// Where a launch goes: to a stream, or to the end of a chain.
+struct LaunchTo {
+    cudaStream_t s = nullptr;
+    GraphChain* chain = nullptr;
+    LaunchTo(cudaStream_t stream) : s(stream) {}
+    LaunchTo(GraphChain& c) : chain(&c) {}
+};
+
+template <class... P, size_t... I>
+void add_kernel(GraphChain& c, bool dependent, void (*k)(P...), unsigned grid, int bs, size_t smem, std::tuple<P...>& args,
+                std::index_sequence<I...>) {
+    void* params[] = {&std::get<I>(args)...};
+    cudaGraphNodeParams p{};
+    p.type = cudaGraphNodeTypeKernel;
+    p.kernel.func = (void*)k;
+    p.kernel.gridDim = dim3(grid);
+    p.kernel.blockDim = dim3(bs);
+    p.kernel.sharedMemBytes = (unsigned)smem;
+    p.kernel.kernelParams = params;
+    cudaGraphEdgeData edge{};
+    if (dependent) {
+        edge.from_port = cudaGraphKernelNodePortProgrammatic;
+        edge.type = cudaGraphDependencyTypeProgrammatic;
+    }
+    cudaGraphNode_t node;
+    GEO_CUDA(cudaGraphAddNode_v2(&node, c.g, c.last ? &c.last : nullptr, c.last ? &edge : nullptr, c.last ? 1 : 0, &p));
+    c.last = node;
+}
+
+// Launches k; in a chain with programmatic dependent launch when `dependent`: its blocks may
+// start, up to their griddepcontrol.wait, while the kernel before it still runs. Only for
+// kernels of the loop: k_patch reads the operator's element data before its wait, which
+// must not be the output of the kernel before it.
 template <class... P, class... A>
-void launch_dependent(bool dependent, void (*k)(P...), unsigned grid, int bs, size_t smem, cudaStream_t s, A... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(bs);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = dependent ? 1 : 0;
-    GEO_CUDA(cudaLaunchKernelEx(&cfg, k, P(args)...));
+void launch_kernel(LaunchTo to, bool dependent, void (*k)(P...), unsigned grid, int bs, size_t smem, A... args) {
+    std::tuple<P...> a{P(args)...};
+    if (to.chain) {
+        add_kernel(*to.chain, dependent, k, grid, bs, smem, a, std::index_sequence_for<P...>{});
+        return;
+    }
+    std::apply([&](auto&... v) { k<<<grid, bs, smem, to.s>>>(v...); }, a);
+    GEO_CUDA(cudaGetLastError());
 }
 
 // Blocks of the patch kernel: the resident ones, or one per patch.
 unsigned patch_blocks(const geo_op* op, int slot) { return (unsigned)std::min(op->patch_grid[slot], op->n_patches); }
 
 template <class K, class T, int MODE>
-void launch_patch(const geo_op* op, int slot, cudaStream_t s, const T* qd, const PatchArgs<T>& pa, bool dependent = false) {
+void launch_patch(const geo_op* op, int slot, LaunchTo to, const T* qd, const PatchArgs<T>& pa, bool dependent = false) {
     PatchView v = view(op);
     v.own_bulk = op->own_bulk[slot];
     with_patch_kernel<K, T, MODE>(op->nbuf[slot], op->halo[slot], [&](auto k) {
-        launch_dependent(dependent, k, patch_blocks(op, slot), kPatchBS, op->patch_smem[slot], s, v, qd,
-                         (T)op->cl, (T)op->cm, pa);
+        launch_kernel(to, dependent, k, patch_blocks(op, slot), kPatchBS, op->patch_smem[slot], v, qd, (T)op->cl,
+                      (T)op->cm, pa);
     });
 }
 
@@ -1057,21 +1091,21 @@ unsigned update_blocks(const geo_op* op, int slot) {
 // The node update of the PCG loop: the halo-mode kernel when the patch kernel runs
 // in halo mode.
 template <class K, class T, bool MIXED>
-void launch_update(const geo_op* op, cudaStream_t s, const NodeArgs<T>& na, bool dependent = false) {
+void launch_update(const geo_op* op, LaunchTo to, const NodeArgs<T>& na, bool dependent = false) {
     constexpr int slot = std::is_same<T, double>::value ? 0 : 1;
     const unsigned g = update_blocks(op, slot);
-    launch_dependent(dependent, op->halo[slot] ? k_pcg_update_halo<T, K::DPN, MIXED> : k_pcg_update<T, K::DPN, MIXED>, g,
-                     kNodeBS, 0, s, na);
+    launch_kernel(to, dependent, op->halo[slot] ? k_pcg_update_halo<T, K::DPN, MIXED> : k_pcg_update<T, K::DPN, MIXED>, g,
+                  kNodeBS, 0, na);
 }
 
-// Enqueues one PCG iteration (patch kernel in PCG mode + node update) of the loop's graph.
+// Adds one PCG iteration (patch kernel in PCG mode + node update) to the loop's graph.
 template <class K, class T, bool MIXED>
-void enqueue_iteration(geo_op* op, cudaStream_t s, const PatchArgs<T>& pa, const NodeArgs<T>& na) {
+void add_iteration(geo_op* op, GraphChain& c, const PatchArgs<T>& pa, const NodeArgs<T>& na) {
     constexpr bool dbl = std::is_same<T, double>::value;
     const T* qd = dbl ? (const T*)op->qd64.p : (const T*)op->qd32.p;
     const bool dependent = op->ndof <= kDependentDofs;
-    launch_patch<K, T, MODE_PCG>(op, dbl ? 0 : 1, s, qd, pa, dependent);
-    launch_update<K, T, MIXED>(op, s, na, dependent);
+    launch_patch<K, T, MODE_PCG>(op, dbl ? 0 : 1, c, qd, pa, dependent);
+    launch_update<K, T, MIXED>(op, c, na, dependent);
 }
 
 // Kernel arguments of the PCG loop over the operator's workspace (FP64 mode: r, q,
@@ -1182,35 +1216,12 @@ cudaGraph_t add_conditional(cudaGraph_t g, const cudaGraphNode_t* dep, cudaGraph
     return p.conditional.phGraph_out[0];
 }
 
-// Captures what enqueue() launches on s into g and returns its last node.
-template <class F>
-cudaGraphNode_t capture_into(cudaGraph_t g, cudaStream_t s, F&& enqueue) {
-    GEO_CUDA(cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    cudaGraphNode_t last = nullptr;
-    cudaGraph_t out = nullptr;
-    try {
-        enqueue();
-        cudaStreamCaptureStatus status;
-        const cudaGraphNode_t* deps = nullptr;
-        size_t n_deps = 0;
-        GEO_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &deps, &n_deps));
-        GEO_CHECK_ARG(n_deps == 1, "PCG loop capture: one stream");
-        last = deps[0];
-    } catch (...) {
-        cudaStreamEndCapture(s, &out);
-        throw;
-    }
-    GEO_CUDA(cudaStreamEndCapture(s, &out));
-    return last;
-}
-
 // The PCG loop as one graph: WHILE (again) { kChunk iterations, k_pcg_decide, mixed: IF
 // (refresh) { the FP64 refresh } }. The kernels of a chunk turn into no-ops once the state
 // says done or refresh. The host used to read the state after each chunk and to launch the
 // refreshes (12 us each time): per iteration, before and now: 6^3 FP64 11.6 -> 11.4 us,
 // 16^3 mixed 15.1 -> 13.5, elastic 8^3 mixed 17.7 -> 16.2, 48x48x32 mixed 23.5 -> 22.6.
 cudaGraphExec_t build_loop(geo_op* op, bool mixed, const PcgLaunchArgs& la) {
-    cudaStream_t s = op->ctx->stream;
     struct Graph {
         cudaGraph_t g = nullptr;
         ~Graph() {
@@ -1220,19 +1231,16 @@ cudaGraphExec_t build_loop(geo_op* op, bool mixed, const PcgLaunchArgs& la) {
     GEO_CUDA(cudaGraphCreate(&graph.g, 0));
     cudaGraphConditionalHandle again, refresh = 0;
     GEO_CUDA(cudaGraphConditionalHandleCreate(&again, graph.g, 1, cudaGraphCondAssignDefault));
-    const cudaGraph_t body = add_conditional(graph.g, nullptr, again, cudaGraphCondTypeWhile);
-    if (mixed) GEO_CUDA(cudaGraphConditionalHandleCreate(&refresh, body, 0, cudaGraphCondAssignDefault));
-    const cudaGraphNode_t decided = capture_into(body, s, [&] {
-        with_kernels(op, [&](auto k64, auto k32) {
-            for (int i = 0; i < kChunk; ++i) {
-                if (mixed) enqueue_iteration<decltype(k32), float, true>(op, s, la.p32, la.n32);
-                else enqueue_iteration<decltype(k64), double, false>(op, s, la.p64, la.n64);
-            }
-        });
-        if (mixed) k_pcg_decide<true><<<1, kNodeBS, 0, s>>>(op->state.p, la.p32.part_in, la.p32.n_in, again, refresh);
-        else k_pcg_decide<false><<<1, kNodeBS, 0, s>>>(op->state.p, la.p64.part_in, la.p64.n_in, again, refresh);
-        check_launch(op->ctx, "PCG loop");
+    GraphChain body{add_conditional(graph.g, nullptr, again, cudaGraphCondTypeWhile)};
+    if (mixed) GEO_CUDA(cudaGraphConditionalHandleCreate(&refresh, body.g, 0, cudaGraphCondAssignDefault));
+    with_kernels(op, [&](auto k64, auto k32) {
+        for (int i = 0; i < kChunk; ++i) {
+            if (mixed) add_iteration<decltype(k32), float, true>(op, body, la.p32, la.n32);
+            else add_iteration<decltype(k64), double, false>(op, body, la.p64, la.n64);
+        }
     });
+    if (mixed) launch_kernel(body, false, k_pcg_decide<true>, 1, kNodeBS, 0, op->state.p, la.p32.part_in, la.p32.n_in, again, refresh);
+    else launch_kernel(body, false, k_pcg_decide<false>, 1, kNodeBS, 0, op->state.p, la.p64.part_in, la.p64.n_in, again, refresh);
     if (mixed) {
         NodeArgs<float> n32 = la.n32;
         n32.again = again;
@@ -1242,16 +1250,13 @@ cudaGraphExec_t build_loop(geo_op* op, bool mixed, const PcgLaunchArgs& la) {
         ra.err = &op->state.p->err;
         if (op->halo[0]) ra.halo = op->halo64.p;  // fixed-order foreign sums: bit-reproducible refresh
         const unsigned ng = node_blocks(op, 1, op->ndof);
-        capture_into(add_conditional(body, &decided, refresh, cudaGraphCondTypeIf), s, [&] {
-            k_refresh_flush<<<ng, kNodeBS, 0, s>>>(n32);
-            with_kernels(op, [&](auto k64, auto) {
-                launch_patch<decltype(k64), double, MODE_FREE>(op, 0, s, op->qd64.p, ra);
-            });
-            if (op->halo[0]) k_refresh_residual_halo<<<ng, kNodeBS, 0, s>>>(n32);
-            else k_refresh_residual<<<ng, kNodeBS, 0, s>>>(n32);
-            k_refresh_rescale<<<ng, kNodeBS, 0, s>>>(n32);
-            check_launch(op->ctx, "refresh");
+        GraphChain rest{add_conditional(body.g, &body.last, refresh, cudaGraphCondTypeIf)};
+        launch_kernel(rest, false, k_refresh_flush, ng, kNodeBS, 0, n32);
+        with_kernels(op, [&](auto k64, auto) {
+            launch_patch<decltype(k64), double, MODE_FREE>(op, 0, rest, op->qd64.p, ra);
         });
+        launch_kernel(rest, false, op->halo[0] ? k_refresh_residual_halo : k_refresh_residual, ng, kNodeBS, 0, n32);
+        launch_kernel(rest, false, k_refresh_rescale, ng, kNodeBS, 0, n32);
     }
     cudaGraphExec_t exec = nullptr;
     GEO_CUDA(cudaGraphInstantiate(&exec, graph.g, 0));
@@ -1277,8 +1282,8 @@ int solve_new(geo_op* op, const geo_cg_opts& o, geo_solver_stats* st) {
     const unsigned ng = node_blocks(op, mixed ? 1 : 0, op->ndof);
     GEO_CUDA(cudaEventRecord(ctx->ev0, s));
     pcg_start(op, mixed, init, la);
-    // (re)build the loop's graph when a buffer that it captured has moved: an FP64 solve, or
-    // the timing of one, grows w64, which the mixed loop's refresh works in
+    // (re)build the loop's graph when a buffer in it has moved: an FP64 solve, or the timing of
+    // one, grows w64, which the mixed loop's refresh works in
     const int pi = mixed ? 1 : 0;
     const void* on[2] = {op->w64.p, mixed ? op->w32.p : nullptr};
     if (!op->loop[pi] || op->loop_on[pi][0] != on[0] || op->loop_on[pi][1] != on[1]) {
